@@ -21,7 +21,7 @@ from .hadamard import get_hadK
 
 F16, BF16 = 0, 1
 GEMM_AUTO, GEMM_TCGEN05, GEMM_MMA_SYNC, GEMM_STREAM, GEMM_STREAM_SPLITK, GEMM_TCGEN05_DIRECT = 0, 1, 2, 3, 4, 5
-GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_DECODE_TC = 6, 7, 8
+GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_DECODE_TC, GEMM_GROUP_F8, GEMM_AUTO_WORKSPACE = 6, 7, 8, 9, 10
 
 
 def _check(cond: bool, msg: str) -> None:
@@ -312,8 +312,11 @@ _SCRATCH: dict = {}
 
 
 def _scratch(device, stream: int, nbytes: int):
-    """Uninitialised scratch for the int8-operand GEMM (the expanded operands), one per (device, stream); kept
-    apart from the zeroed split-K workspace, whose counters it would overwrite."""
+    """Uninitialised scratch for the GEMMs that expand their operands first, one per (device, stream); kept apart from the
+    zeroed split-K workspace, whose counters it would overwrite.  A launch that is being recorded into a graph gets memory
+    of the graph's own instead: the shared buffer is replaced when a larger call comes, the graph would go on using it."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
     key = (str(device), stream)
     ws = _SCRATCH.get(key)
     if ws is None or ws.numel() < nbytes:
@@ -338,11 +341,12 @@ def gemm_i4_dequant(A, B, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=Non
     lib = _lib.load()
     with _guard(A.device):
         stream = _stream(A)
-        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, algo)
+        # zero-points rule out the kernel that AUTO could use more workspace for
+        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if algo == GEMM_AUTO and A_zero is None else algo)
         resolved = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
         if not need:
             ws = None
-        elif resolved in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR):
+        elif M > 64 or resolved in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_GROUP_F8):
             ws = _scratch(A.device, stream, need)          # expanded operands: any contents
         else:
             ws = _workspace(A.device, stream, need)        # split-K: zeroed counters, left zeroed

@@ -79,6 +79,13 @@ int gemm_decode_tc_status(int *);
 int gemm_decode_tc_status_clear();
 int gemm_decode_tc_wait_profile(unsigned long long *);
 
+bool gemm_group_f8_supported(long M, long N, long K);
+size_t gemm_group_f8_workspace_bytes(long M, long N, long K);
+int launch_gemm_group_f8(const uint8_t *, const uint8_t *, const void *, const void *, const void *, void *, long, long, long, long, long,
+                         int, void *, cudaStream_t);
+int gemm_group_f8_status(int *);
+int gemm_group_f8_status_clear();
+
 int gemm_tcgen05_status(int *);
 int gemm_tcgen05_wait_profile(unsigned long long *);
 int gemm_tcgen05_status_clear();
@@ -267,6 +274,11 @@ static int pick_stream(long M, long N, long K) {
     return stream_splits(M, N, K) > 1 ? FLH_B200_GEMM_STREAM_SPLITK : FLH_B200_GEMM_STREAM;
 }
 
+// Prefill batches with group-128 scales for which expanding both operands first pays for itself (measured on B200).
+static bool group_f8_pays(long M, long N, long K, long a_group, long b_group) {
+    return (a_group < b_group ? a_group : b_group) == 128 && K > 128 && M >= 256 && gemm_group_f8_supported(M, N, K);
+}
+
 int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) {
     if ((a_group < b_group ? a_group : b_group) < 128) return FLH_B200_GEMM_MMA_SYNC;    // K-groups of 32 / 64
     if (M <= 64) return decode_tc_pays(M, N, K, a_group) ? FLH_B200_GEMM_DECODE_TC : pick_stream(M, N, K);
@@ -278,7 +290,9 @@ int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) 
 }
 
 size_t flh_b200_gemm_workspace_bytes(long M, long N, long K, long a_group, long b_group, int algo) {
+    if (algo == FLH_B200_GEMM_AUTO_WORKSPACE) algo = group_f8_pays(M, N, K, a_group, b_group) ? FLH_B200_GEMM_GROUP_F8 : FLH_B200_GEMM_AUTO;
     if (algo == FLH_B200_GEMM_AUTO) algo = flh_b200_gemm_pick_algo(M, N, K, a_group, b_group);
+    if (algo == FLH_B200_GEMM_GROUP_F8) return gemm_group_f8_supported(M, N, K) ? gemm_group_f8_workspace_bytes(M, N, K) : 0;
     if (algo == FLH_B200_GEMM_TCGEN05_I8 || algo == FLH_B200_GEMM_TCGEN05_I8_PAIR) return gemm_i8_workspace_bytes(M, N, K);
     if (algo == FLH_B200_GEMM_DECODE_TC) return M <= 64 ? gemm_decode_tc_workspace_bytes(M, N, K) : 0;
     if (algo != FLH_B200_GEMM_STREAM_SPLITK || M > 64) return 0;
@@ -324,6 +338,10 @@ int flh_b200_gemm_i4_dequant(const uint8_t *A, const uint8_t *B, const void *a_s
         if ((algo == FLH_B200_GEMM_TCGEN05_I8 || algo == FLH_B200_GEMM_TCGEN05_I8_PAIR) &&
             (!workspace || workspace_bytes < gemm_i8_workspace_bytes(M, N, K) || (reinterpret_cast<uintptr_t>(workspace) & 255)))
             algo = FLH_B200_GEMM_TCGEN05;
+        // group scales: the expanding kernel needs scratch that nobody has to hand over
+        if (algo == FLH_B200_GEMM_TCGEN05 && !a_zero && group_f8_pays(M, N, K, a_group, b_group) && workspace &&
+            workspace_bytes >= gemm_group_f8_workspace_bytes(M, N, K) && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0)
+            algo = FLH_B200_GEMM_GROUP_F8;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     switch (algo) {
@@ -365,6 +383,14 @@ int flh_b200_gemm_i4_dequant(const uint8_t *A, const uint8_t *B, const void *a_s
             FLH_REQUIRE(algo == FLH_B200_GEMM_TCGEN05_I8 || N % 256 == 0, FLH_B200_EINVAL, "the two-CTA kernel needs N %% 256 == 0 (got %ld)", N);
             return launch_gemm_i8(A, B, nullptr, a_scale, a_zero, b_scale, b_rowsum, bias, D, M, N, K, out_dtype,
                                   algo == FLH_B200_GEMM_TCGEN05_I8_PAIR, workspace, s);
+        }
+        case FLH_B200_GEMM_GROUP_F8: {
+            FLH_REQUIRE(gmin == 128 && !a_zero, FLH_B200_EINVAL, "the fp8 group kernel takes groups of 128 without zero-points");
+            FLH_REQUIRE(gemm_group_f8_supported(M, N, K), FLH_B200_EINVAL, "the fp8 group kernel needs N %% 256 == 0 (got %ld)", N);
+            const size_t need = gemm_group_f8_workspace_bytes(M, N, K);
+            FLH_REQUIRE(workspace && workspace_bytes >= need, FLH_B200_EINVAL, "the fp8 group kernel needs %zu bytes of workspace (got %zu)", need, workspace_bytes);
+            FLH_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, FLH_B200_EALIGN, "workspace must be 256-byte aligned");
+            return launch_gemm_group_f8(A, B, a_scale, b_scale, bias, D, M, N, K, a_group, b_group, out_dtype, workspace, s);
         }
         case FLH_B200_GEMM_TCGEN05_DIRECT:
             return launch_gemm_tcgen05(A, B, a_scale, a_zero, b_scale, b_rowsum, bias, D, M, N, K, a_group, b_group, out_dtype, 1, s);
@@ -443,6 +469,9 @@ int flh_b200_gemm_status(int *out) {
     rc = gemm_i8_status(out);
     if (rc) return rc;
     if (out[0]) return gemm_i8_status_clear();
+    rc = gemm_group_f8_status(out);
+    if (rc) return rc;
+    if (out[0]) return gemm_group_f8_status_clear();
     rc = quant_token_factor_status(out);
     if (rc) return rc;
     if (out[0]) return quant_token_factor_status_clear();

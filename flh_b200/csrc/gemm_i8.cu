@@ -16,7 +16,7 @@
 // The int32 dot product is 256 * sum(qa qw); the factor is folded back exactly in the epilogue.
 // Every wait is bounded (two seconds) and reports through the same status word as the other GEMM kernels.
 #include "tc_common.cuh"
-#include <cooperative_groups.h>
+#include "tc_pair.cuh"
 
 namespace flh {
 namespace {
@@ -34,34 +34,6 @@ __device__ __forceinline__ bool wait_i8(uint32_t bar, uint32_t parity, volatile 
     return mbar_wait_status(g_status_i8, bar, parity, abort_flag, code, waited);
 }
 
-// ---- cluster helpers (PAIR) -------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
-    uint32_t raddr;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(bar), "r"(rank));
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(raddr) : "memory");
-}
-// TMA tile load of a CTA of a pair whose completion is counted on the barrier at the same offset in CTA 0
-__device__ __forceinline__ void tma_load_2d_to_leader(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
-    uint32_t rbar;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(rbar) : "r"(bar));
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(rbar) : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    const uint16_t mask = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask) : "memory");
-}
 template <bool PAIR>
 __device__ __forceinline__ void tc_mma_i8_plain(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
     if (PAIR)
@@ -283,48 +255,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ---- host side -----------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-    return fn;
-}
-
-// rows x K bytes, row-major; box = box_rows x 128 bytes written with the 128-byte swizzle; rows past the end read as 0.
-int make_map_i8(CUtensorMap *map, const uint8_t *ptr, long rows, long K, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(FLH_B200_EUNSUPPORTED, "cuTensorMapEncodeTiled is not available from this driver");
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K};
-    cuuint32_t box[2] = {128u, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1u, 1u};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(FLH_B200_EINVAL, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-    return 0;
-}
-
-int device_sms() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = kNumSMs;
-    }
-    return sms;
-}
-
 template <int BN, bool U, bool PAIR>
 int launch_i8(const CUtensorMap &ma, const CUtensorMap &mb, const I8Params &p, cudaStream_t stream) {
     using Plan = I8Plan<BN, PAIR>;
@@ -335,7 +265,7 @@ int launch_i8(const CUtensorMap &ma, const CUtensorMap &mb, const I8Params &p, c
     const int tile_m = PAIR ? 2 * BM : BM;
     q.m_blocks = (p.M + tile_m - 1) / tile_m;
     q.num_tiles = q.m_blocks * (p.N / BN);
-    const int sms = device_sms();
+    const int sms = tc_device_sms();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.blockDim = dim3(Plan::kThreads);
@@ -374,7 +304,7 @@ int launch_expand_i4(const uint8_t *packed, long rows, long K, uint8_t *out, cud
     const long n16 = rows * K / 32;                            // 16-byte packed chunks
     if (n16 == 0) return 0;
     long grid = (n16 + 255) / 256;
-    const long cap = 8L * device_sms();
+    const long cap = 8L * tc_device_sms();
     if (grid > cap) grid = cap;
     expand_i4_kernel<<<(unsigned)grid, 256, 0, stream>>>(reinterpret_cast<const uint4 *>(packed), reinterpret_cast<uint4 *>(out), n16);
     return cuda_status(cudaGetLastError(), "expand_i4 launch");
@@ -405,16 +335,16 @@ int launch_gemm_i8(const uint8_t *A, const uint8_t *B, const uint8_t *B8, const 
     p.out_bf16 = out_dtype == FLH_B200_BF16;
     const bool u = a_zero != nullptr;
     CUtensorMap ma, mb;
-    rc = make_map_i8(&ma, ea, M, K, BM);
+    rc = make_map_bytes(&ma, ea, M, K, BM);
     if (rc) return rc;
     if (pair) {
         if (N % 256 != 0) return fail(FLH_B200_EINVAL, "the two-CTA kernel needs N %% 256 == 0 (got %ld)", N);
-        rc = make_map_i8(&mb, eb, N, K, 128);
+        rc = make_map_bytes(&mb, eb, N, K, 128);
         if (rc) return rc;
         return u ? launch_i8<256, true, true>(ma, mb, p, stream) : launch_i8<256, false, true>(ma, mb, p, stream);
     }
     const int bn = (N % 256 == 0) ? 256 : 128;
-    rc = make_map_i8(&mb, eb, N, K, bn);
+    rc = make_map_bytes(&mb, eb, N, K, bn);
     if (rc) return rc;
     if (bn == 256) return u ? launch_i8<256, true, false>(ma, mb, p, stream) : launch_i8<256, false, false>(ma, mb, p, stream);
     return u ? launch_i8<128, true, false>(ma, mb, p, stream) : launch_i8<128, false, false>(ma, mb, p, stream);

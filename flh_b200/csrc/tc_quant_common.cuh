@@ -25,13 +25,6 @@ __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
     asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
     return r;
 }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-
 // A = G (or diag(G, G) when two token rows share an MMA: R == 2) as a K-major tcgen05 operand with the 128-byte swizzle:
 // element (m, k) lies in K atom kb = k / 64 at (kb * Mtot / 8 + m / 8) * 1024, row m % 8 of 128 bytes, 16-byte chunk
 // ((k % 64) / 8) ^ (m % 8).  G[p'][p] = S[a'][a] * (-1)^popc(b' & b) with p = a * B + b (B a power of two, S the kfac x kfac

@@ -53,6 +53,9 @@ extern "C" {
                                           N % 256 == 0                                                         */
 #define FLH_B200_GEMM_DECODE_TC 8 /* M <= 64 on the tensor cores with the operands swapped (weights on the MMA's M side),
                                     K-ranges balanced across CTAs; needs zero-initialised workspace like split-K */
+#define FLH_B200_GEMM_GROUP_F8 9 /* prefill batches with group-128 scales and no zero-points: operands expanded to e4m3 in the
+                                    workspace, two-CTA tcgen05 kernel with exact binary32 group sums; N % 256 == 0 */
+#define FLH_B200_GEMM_AUTO_WORKSPACE 10 /* only for flh_b200_gemm_workspace_bytes: the most workspace AUTO can make use of */
 
 int flh_b200_version(void);
 const char *flh_b200_last_error(void);
@@ -204,6 +207,9 @@ int flh_b200_weight_rowsum(const uint8_t *B, long N, long K, long group, int32_t
  *   The int8-operand kernels (TCGEN05_I8, TCGEN05_I8_PAIR; a_group = b_group = K only) write the expanded
  *   operands, (M + N) * K bytes, into the workspace; it needs no initial contents, results are bit-identical
  *   to the other kernels, and launches that share a workspace must not overlap on the GPU.
+ *   GROUP_F8 (groups of 128, a_zero = NULL, N % 256 == 0) likewise: the e4m3 operands and the scales in binary32, results
+ *   bit-identical to TCGEN05.  AUTO takes it for prefill batches when it is handed the bytes that
+ *   flh_b200_gemm_workspace_bytes(.., FLH_B200_GEMM_AUTO_WORKSPACE) asks for, and TCGEN05 when it is not.
  * Replaces flhDenseLayerGEMM_i4_o16 (flh/kernels/gemm_and_dequant_i4.cu:471-508) and
  * flhDenseLayerGEMM_i4_o16_gs (flh/kernels/gemm_and_dequant_i4_gs.h); bound as
  * gemm_i4_dequant_o16(_gs) (flh/cuda/flh_cuda_bindings.cpp:75-113, 253-299). */

@@ -1,0 +1,73 @@
+"""GPU parity of the fp8 group-scale GEMM and of the ring decode GEMM against the CPU oracle, at the edges of their tiles."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import rs
+from oracle import oracle as O
+from test_gpu_gemm import _dev, make_case, run_case
+
+pytestmark = pytest.mark.gpu
+F8, RING, AUTO = 9, 11, 0
+
+
+@pytest.fixture(autouse=True)
+def _status_clean(cuda):
+    yield
+    torch.cuda.synchronize()
+    st = cuda.gemm_status()
+    assert st[0] == 0, f"a bounded wait ran out: code {st[0]} in CTA {st[1]}"
+
+
+# one row, both sides of a 256-row tile, a ragged last tile; one K-group, more groups than scale slots, a count that is no
+# multiple of eight; more tiles than resident pairs; every scale layout
+@pytest.mark.parametrize("m,n,k", [(1, 256, 128), (255, 256, 256), (257, 512, 1024), (515, 1280, 1408), (300, 19200, 256), (700, 768, 11008)])
+@pytest.mark.parametrize("mode", [(128, 128, False), (128, 0, False), (0, 128, False)])
+def test_group_f8_is_bit_exact(cuda, m, n, k, mode):
+    run_case(cuda, F8, make_case(m + n + k, m, n, k, *mode, bias=m == 257), bf16=m == 515)
+
+
+@pytest.mark.parametrize("a,b", [(0x88, 0x88), (0x88, 0x77), (0x77, 0x77)])
+def test_group_f8_extreme_codes(cuda, a, b):
+    """Every code at an end of its range: the largest group sums (8192 units), exact in the fp8 tensor core's accumulator."""
+    ap, bp, sa, sb, _, _ = make_case(7, 300, 512, 1024, 128, 128, False, neg_scales=True)
+    ap[:], bp[:] = a, b
+    run_case(cuda, F8, (ap, bp, sa, sb, None, None))
+
+
+def test_group_f8_needs_its_workspace_and_auto_does_without(cuda):
+    lib, m, n, k = cuda._lib.load(), 300, 512, 1024
+    case = make_case(11, m, n, k, 128, 128, False)
+    run_case(cuda, AUTO, case)
+    A, B, SA, SB = (_dev(t) for t in case[:4])
+    D = torch.empty(m, n, dtype=torch.float16, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    call = lambda algo, ws, nbytes: lib.flh_b200_gemm_i4_dequant(A.data_ptr(), B.data_ptr(), SA.data_ptr(), None, SB.data_ptr(), None, None, D.data_ptr(),
+                                                                 m, n, k, 128, 128, 0, algo, ws, nbytes, s)
+    need = lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, F8)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    assert call(F8, None, 0) != 0 and call(F8, ws.data_ptr(), need - 1) != 0
+    want = O.gemm_i4_dequant(*case[:4]).view(np.uint16)
+    for w, nbytes in ((None, 0), (ws.data_ptr(), need - 1), (ws.data_ptr(), need)):
+        D.zero_()
+        assert call(AUTO, w, nbytes) == 0
+        assert np.array_equal(D.cpu().numpy().view(np.uint16), want)
+
+
+def test_group_f8_scratch_of_a_captured_call_outlives_a_larger_call(cuda):
+    """A recorded launch keeps its own scratch: a later, larger call on the same stream must not take it away."""
+    small, large = make_case(21, 300, 512, 1024, 128, 128, False), make_case(22, 600, 1024, 2048, 128, 128, False)
+    t = [_dev(x) for x in small[:4]]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        cuda.gemm_i4_dequant(*t)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            d = cuda.gemm_i4_dequant(*t)
+        run_case(cuda, AUTO, large)
+        junk = [torch.full((4 << 20,), 255, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        g.replay()
+        torch.cuda.synchronize()
+    assert np.array_equal(d.cpu().numpy().view(np.uint16), O.gemm_i4_dequant(*small[:4]).view(np.uint16))
+    del junk
