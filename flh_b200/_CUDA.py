@@ -21,7 +21,7 @@ from .hadamard import get_hadK
 
 F16, BF16 = 0, 1
 GEMM_AUTO, GEMM_TCGEN05, GEMM_MMA_SYNC, GEMM_STREAM, GEMM_STREAM_SPLITK, GEMM_TCGEN05_DIRECT = 0, 1, 2, 3, 4, 5
-GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_DECODE_TC, GEMM_GROUP_F8, GEMM_AUTO_WORKSPACE = 6, 7, 8, 9, 10
+GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_DECODE_TC, GEMM_GROUP_F8, GEMM_AUTO_WORKSPACE, GEMM_DECODE_RING = 6, 7, 8, 9, 10, 11
 
 
 def _check(cond: bool, msg: str) -> None:
@@ -341,8 +341,9 @@ def gemm_i4_dequant(A, B, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=Non
     lib = _lib.load()
     with _guard(A.device):
         stream = _stream(A)
-        # zero-points rule out the kernel that AUTO could use more workspace for
-        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if algo == GEMM_AUTO and A_zero is None else algo)
+        # what AUTO can use depends on the zero-points only where there are group scales: those keep the kernels without workspace of that kind
+        auto = algo == GEMM_AUTO and not (A_zero is not None and min(ag, bg) < K)
+        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if auto else algo)
         resolved = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
         if not need:
             ws = None

@@ -79,6 +79,11 @@ int gemm_decode_tc_status(int *);
 int gemm_decode_tc_status_clear();
 int gemm_decode_tc_wait_profile(unsigned long long *);
 
+bool gemm_decode_ring_supported(long M, long N, long K, bool grouped, bool zero);
+int launch_gemm_decode_ring(const uint8_t *, const uint8_t *, const void *, const void *, const void *, const int32_t *, const void *, void *,
+                            long, long, long, long, long, int, cudaStream_t);
+int gemm_decode_ring_status(int *);
+int gemm_decode_ring_status_clear();
 bool gemm_group_f8_supported(long M, long N, long K);
 size_t gemm_group_f8_workspace_bytes(long M, long N, long K);
 int launch_gemm_group_f8(const uint8_t *, const uint8_t *, const void *, const void *, const void *, void *, long, long, long, long, long,
@@ -289,7 +294,23 @@ int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) 
     return FLH_B200_GEMM_TCGEN05;
 }
 
+// Decode shapes for which the ring kernel is the faster one (B200, weights from HBM, us, the kernel pick_algo names -> ring):
+//   no group scales, 16 tokens: 4096 -> 12288 11.6 -> 9.4, 4096 -> 4096 8.6 -> 5.1, 11008 -> 4096 13.5 -> 7.7, 8192 -> 28672
+//   35.0 -> 26.6; 64 tokens: 4096 -> 4096 18.1 -> 10.2, but 11008 -> 4096 19.9 -> 20.7 and 8192 -> 28672 48.5 -> 57.5 (its
+//   mma.sync rate is the limit there): above 32 tokens for weights below 20 MiB;
+//   group scales, 16 tokens: 4096 -> 4096 9.0 -> 5.5, 11008 -> 4096 15.3 -> 11.0, 8192 -> 28672 43.1 -> 39.0; 32 tokens: 12.0 -> 7.5,
+//   21.0 -> 14.9, but 55.3 -> 57.8: above 16 tokens for weights below 64 MiB; 64 tokens: never.  Where the plain streaming
+//   kernel is what AUTO ran, AUTO's results are a single binary32 chain bit for bit and stay so.
+static bool decode_ring_pays(long M, long N, long K, long a_group, long b_group, bool zero) {
+    const bool grouped = (a_group < b_group ? a_group : b_group) < K;
+    if (!gemm_decode_ring_supported(M, N, K, grouped, zero)) return false;
+    const double mib = (double)N * (double)K / 2.0 / (1 << 20);
+    if (!grouped) return M <= 32 || mib < 20.0;
+    return (M <= 16 || (M <= 32 && mib < 64.0)) && flh_b200_gemm_pick_algo(M, N, K, a_group, b_group) != FLH_B200_GEMM_STREAM;
+}
+
 size_t flh_b200_gemm_workspace_bytes(long M, long N, long K, long a_group, long b_group, int algo) {
+    if (algo == FLH_B200_GEMM_AUTO_WORKSPACE && decode_ring_pays(M, N, K, a_group, b_group, false)) return 0;
     if (algo == FLH_B200_GEMM_AUTO_WORKSPACE) algo = group_f8_pays(M, N, K, a_group, b_group) ? FLH_B200_GEMM_GROUP_F8 : FLH_B200_GEMM_AUTO;
     if (algo == FLH_B200_GEMM_AUTO) algo = flh_b200_gemm_pick_algo(M, N, K, a_group, b_group);
     if (algo == FLH_B200_GEMM_GROUP_F8) return gemm_group_f8_supported(M, N, K) ? gemm_group_f8_workspace_bytes(M, N, K) : 0;
@@ -324,6 +345,10 @@ int flh_b200_gemm_i4_dequant(const uint8_t *A, const uint8_t *B, const void *a_s
         return launch_gemm_mma_tile_gs(A, B, a_scale, a_zero, b_scale, b_rowsum, bias, D, M, N, K, a_group, b_group, (int)gmin,
                                        out_dtype, static_cast<cudaStream_t>(stream));
     }
+    const bool grouped = gmin < K;
+    // (it reads the scales of two groups as one word)
+    const bool words = ((reinterpret_cast<uintptr_t>(a_scale) | reinterpret_cast<uintptr_t>(b_scale)) & 3) == 0;
+    if (algo == FLH_B200_GEMM_AUTO && words && decode_ring_pays(M, N, K, a_group, b_group, a_zero != nullptr)) algo = FLH_B200_GEMM_DECODE_RING;
     if (algo == FLH_B200_GEMM_AUTO) {
         algo = flh_b200_gemm_pick_algo(M, N, K, a_group, b_group);
         // without (enough) scratch the tensor-core decode kernel gives way to the streaming kernels
@@ -384,6 +409,12 @@ int flh_b200_gemm_i4_dequant(const uint8_t *A, const uint8_t *B, const void *a_s
             return launch_gemm_i8(A, B, nullptr, a_scale, a_zero, b_scale, b_rowsum, bias, D, M, N, K, out_dtype,
                                   algo == FLH_B200_GEMM_TCGEN05_I8_PAIR, workspace, s);
         }
+        case FLH_B200_GEMM_DECODE_RING:
+            FLH_REQUIRE(M <= 64, FLH_B200_EINVAL, "the decode kernel serves M <= 64 (got %ld)", M);
+            FLH_REQUIRE(words, FLH_B200_EALIGN, "the scales must be 4-byte aligned");
+            FLH_REQUIRE(gemm_decode_ring_supported(M, N, K, grouped, a_zero != nullptr), FLH_B200_EUNSUPPORTED,
+                        "the ring kernel does not serve K=%ld with this scale layout", K);
+            return launch_gemm_decode_ring(A, B, a_scale, a_zero, b_scale, b_rowsum, bias, D, M, N, K, a_group, b_group, out_dtype, s);
         case FLH_B200_GEMM_GROUP_F8: {
             FLH_REQUIRE(gmin == 128 && !a_zero, FLH_B200_EINVAL, "the fp8 group kernel takes groups of 128 without zero-points");
             FLH_REQUIRE(gemm_group_f8_supported(M, N, K), FLH_B200_EINVAL, "the fp8 group kernel needs N %% 256 == 0 (got %ld)", N);
@@ -469,6 +500,9 @@ int flh_b200_gemm_status(int *out) {
     rc = gemm_i8_status(out);
     if (rc) return rc;
     if (out[0]) return gemm_i8_status_clear();
+    rc = gemm_decode_ring_status(out);
+    if (rc) return rc;
+    if (out[0]) return gemm_decode_ring_status_clear();
     rc = gemm_group_f8_status(out);
     if (rc) return rc;
     if (out[0]) return gemm_group_f8_status_clear();

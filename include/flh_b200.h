@@ -55,6 +55,9 @@ extern "C" {
                                     K-ranges balanced across CTAs; needs zero-initialised workspace like split-K */
 #define FLH_B200_GEMM_GROUP_F8 9 /* prefill batches with group-128 scales and no zero-points: operands expanded to e4m3 in the
                                     workspace, two-CTA tcgen05 kernel with exact binary32 group sums; N % 256 == 0 */
+#define FLH_B200_GEMM_DECODE_RING 11 /* M <= 64: weights through a TMA ring, mma.sync, K split over the warps of a CTA; no workspace.
+                                     AUTO runs it before what flh_b200_gemm_pick_algo names: without group scales up to 32
+                                     tokens (64 for small weights), with them in place of SPLITK and DECODE_TC up to 16 (32) */
 #define FLH_B200_GEMM_AUTO_WORKSPACE 10 /* only for flh_b200_gemm_workspace_bytes: the most workspace AUTO can make use of */
 
 int flh_b200_version(void);

@@ -71,3 +71,33 @@ def test_group_f8_scratch_of_a_captured_call_outlives_a_larger_call(cuda):
         torch.cuda.synchronize()
     assert np.array_equal(d.cpu().numpy().view(np.uint16), O.gemm_i4_dequant(*small[:4]).view(np.uint16))
     del junk
+
+
+SHAPES = [(128, 128), (64 * 3 * 2, 1152), (256, 2048), (512, 11008), (19200, 384)]   # half a chunk, half a stage, one stage, many; many tiles
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k", SHAPES)
+@pytest.mark.parametrize("asym", [False, True])
+def test_ring_without_group_scales_is_bit_exact(cuda, m, n, k, asym):
+    run_case(cuda, RING, make_case(m + n + k, m, n, k, 0, 0, asym, bias=m == 9), bf16=m == 17)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k", SHAPES)
+@pytest.mark.parametrize("mode", [(128, 128, False), (128, 0, False), (0, 128, False)])
+def test_ring_with_group_scales(cuda, m, n, k, mode):
+    """A warp keeps the binary32 chain of its K-groups and the chains are added: each order of G terms is within
+    G 2^-24 sum |terms| of the exact sum, so two orders differ by at most twice that, and the result by one ulp (2^-10) of its
+    own rounding on top.  The same bits on every run."""
+    ap, bp, sa, sb, _, _ = make_case(m + n + k, m, n, k, *mode)
+    args = [_dev(t) for t in (ap, bp, sa, sb)]
+    d1, d2 = cuda.gemm_i4_dequant(*args, algo=RING), cuda.gemm_i4_dequant(*args, algo=RING)
+    assert torch.equal(d1.view(torch.int16), d2.view(torch.int16))
+    G = k // 128
+    a = np.abs(O.unpack_i4(ap).astype(np.float64)).reshape(m, G, 128) * np.broadcast_to(sa.astype(np.float64), (m, G))[:, :, None]
+    b = np.abs(O.unpack_i4(bp).astype(np.float64)).reshape(n, G, 128) * np.broadcast_to(sb.astype(np.float64), (n, G))[:, :, None]
+    bound = 2 * G * 2.0 ** -24 * (a.reshape(m, k) @ b.reshape(n, k).T)
+    ref = O.gemm_i4_dequant(ap, bp, sa, sb).astype(np.float64)
+    err = np.abs(d1.cpu().numpy().astype(np.float64) - ref)
+    assert (err <= bound + 2.0 ** -10 * np.abs(ref) + 2.0 ** -24).all(), err.max()
