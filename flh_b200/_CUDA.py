@@ -242,15 +242,17 @@ def silu_mul_quant_token_asym_i4(gu, hadamard: bool = True, clip: float = 1.0, e
     return quant_token_asym_i4(silu_mul(gu), hadamard=hadamard, clip=clip, exact=exact)
 
 
-def rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, cur):
+def rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, cur, q_by_token: bool = False):
     """Rotary embedding of q and k + KV-cache write from the merged QKV GEMM output (include/flh_b200.h: flh_b200_rope_kv_f16).
-    qkv f16 [B*S, (nh + 2 nkv) * D] contiguous; cos, sin f32 [S, D/2]; q_out [B, nh, S, D]; caches [B, nkv, T, D] contiguous."""
+    qkv f16 [B*S, (nh + 2 nkv) * D] contiguous; cos, sin f32 [S, D/2]; q_out [B, nh, S, D] (q_by_token: [B, S, nh, D]); caches [B, nkv, T, D] contiguous."""
     _check(qkv.is_cuda and qkv.dtype == torch.float16 and qkv.is_contiguous(), "qkv must be a contiguous CUDA float16 tensor")
     _check(cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous(), "cos / sin must be contiguous float32")
     _check(q_out.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous(), "outputs must be contiguous")
     D = q_out.shape[-1]
     with _guard(qkv.device):
-        _lib.check(_lib.load().flh_b200_rope_kv_f16(_ptr(qkv), _ptr(cos), _ptr(sin), _ptr(q_out), _ptr(k_cache), _ptr(v_cache),
+        lib = _lib.load()
+        fn = lib.flh_b200_rope_kv_by_token_f16 if q_by_token else lib.flh_b200_rope_kv_f16
+        _lib.check(fn(_ptr(qkv), _ptr(cos), _ptr(sin), _ptr(q_out), _ptr(k_cache), _ptr(v_cache),
                                                     B, S, nh, nkv, D, k_cache.shape[2], cur, _stream(qkv)), "rope_kv")
     return q_out
 

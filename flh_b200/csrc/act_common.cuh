@@ -27,6 +27,52 @@ __device__ __forceinline__ float exp32(float t) {
     return __fmul_rn(y, __int_as_float(((int)n + 127) << 23));
 }
 
+// The same values for two gates at once in packed binary32, for finite gates of magnitude 2^-90 and up and, in bfloat16, above
+// -80 (silu2_takes; float16 has no smaller ones, and its quotients below -80 round to -0 either way).  There no step of exp32
+// rounds to a subnormal or overflows:
+//   * rint by adding 1.5 * 2^23, whose low bits then are n for the exponent;
+//   * the quotient by Newton-Raphson on a reciprocal estimate and a final fused residual step (Markstein, IBM J. Res. Dev. 34,
+//     1990): rounded like the division it replaces.  s is a function of one 16-bit value, and the test compares every one.
+// Half the issue slots of the scalar form: the kernel was bound by issue (0.54 of the copy bandwidth), not by memory.
+__device__ __forceinline__ uint64_t dup2(float v) { return pack2(v, v); }
+__device__ __forceinline__ float rcp_estimate(float d) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+}
+__device__ __forceinline__ uint64_t silu2(uint64_t g) {
+    float g0, g1;
+    unpack2(g, g0, g1);
+    const uint64_t t = pack2(fminf(fmaxf(-g0, -87.0f), 80.0f), fminf(fmaxf(-g1, -87.0f), 80.0f));
+    const uint64_t nb = add2(mul2(t, dup2(1.44269504088896341f)), dup2(12582912.0f));
+    const uint64_t n = add2(nb, dup2(-12582912.0f));
+    uint64_t r = fma2(n, dup2(-0.693359375f), t);
+    r = fma2(n, dup2(2.12194440e-4f), r);
+    const uint64_t z = mul2(r, r);
+    uint64_t y = fma2(dup2(1.9875691500e-4f), r, dup2(1.3981999507e-3f));
+    y = fma2(y, r, dup2(8.3334519073e-3f));
+    y = fma2(y, r, dup2(4.1665795894e-2f));
+    y = fma2(y, r, dup2(1.6666665459e-1f));
+    y = fma2(y, r, dup2(5.0000001201e-1f));
+    y = fma2(y, z, r);
+    y = add2(y, dup2(1.0f));
+    // y * 2^n: n goes straight into the exponent (the bits above n of nb leave the word)
+    const uint32_t e0 = (uint32_t)y + ((uint32_t)nb << 23), e1 = (uint32_t)(y >> 32) + ((uint32_t)(nb >> 32) << 23);
+    const uint64_t d = add2(((uint64_t)e1 << 32) | e0, dup2(1.0f));
+    float d0, d1;
+    unpack2(d, d0, d1);
+    uint64_t q = pack2(rcp_estimate(d0), rcp_estimate(d1));
+    const uint64_t nd = mul2(d, dup2(-1.0f));
+    q = fma2(q, fma2(nd, q, dup2(1.0f)), q);                // reciprocal of d
+    const uint64_t a = mul2(g, q);
+    return fma2(fma2(nd, a, g), q, a);
+}
+template <bool BF16>
+__device__ __forceinline__ bool silu2_takes(float g) {
+    const float m = fabsf(g);
+    return m > (BF16 ? 8.0e-28f : 0.0f) && m < 3.0e38f && (!BF16 || g > -80.0f);
+}
+
 // two neighbouring elements at once: g2, u2 hold two 16-bit values each (low half = the lower index)
 template <bool BF16>
 __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g2, uint32_t u2) {
@@ -39,8 +85,13 @@ __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g2, uint32_t u2) {
         const float2 uf = __half22float2(*reinterpret_cast<const __half2 *>(&u2));
         g0 = gf.x; g1 = gf.y; u0 = uf.x; u1 = uf.y;
     }
-    const float s0 = __fdiv_rn(g0, __fadd_rn(1.0f, exp32(-g0)));
-    const float s1 = __fdiv_rn(g1, __fadd_rn(1.0f, exp32(-g1)));
+    float s0, s1;
+    if (silu2_takes<BF16>(g0) && silu2_takes<BF16>(g1)) {
+        unpack2(silu2(pack2(g0, g1)), s0, s1);
+    } else {
+        s0 = __fdiv_rn(g0, __fadd_rn(1.0f, exp32(-g0)));
+        s1 = __fdiv_rn(g1, __fadd_rn(1.0f, exp32(-g1)));
+    }
     if (BF16) {
         const float a0 = __bfloat162float(__float2bfloat16_rn(s0)), a1 = __bfloat162float(__float2bfloat16_rn(s1));
         const __nv_bfloat162 o = __floats2bfloat162_rn(__fmul_rn(a0, u0), __fmul_rn(a1, u1));

@@ -61,7 +61,7 @@ int quant_token_factor_status_clear();
 const char *quant_token_kernel_name(long, long, int, int);
 int launch_silu_mul(const void *, int, long, long, long, void *, cudaStream_t);
 int launch_silu_mul_quant_token_tc(const void *, int, long, long, long, int, const uint32_t *, float, uint8_t *, void *, void *, cudaStream_t);
-int launch_rope_kv(const void *, const float *, const float *, void *, void *, void *, int, int, int, int, int, int, int, cudaStream_t);
+int launch_rope_kv(const void *, const float *, const float *, void *, void *, void *, int, int, int, int, int, int, int, int, cudaStream_t);
 int quant_token_tc_status(int *);
 int launch_gptq_block(const float *, long, const float *, long, const float *, const float *, long, const int *, long, int, int, int,
                       float, float *, long, float *, cudaStream_t);
@@ -100,6 +100,17 @@ static bool is_pow2(long v) { return v > 0 && (v & (v - 1)) == 0; }
 }  // namespace flh
 
 using namespace flh;
+
+static int rope_kv(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
+                         int B, int S, int nh, int nkv, int D, int T, int cur, int q_by_token, void *stream) {
+    FLH_REQUIRE(B >= 0 && S >= 0 && nh > 0 && nkv > 0 && D > 0 && D % 8 == 0, FLH_B200_EINVAL, "bad shape B=%d S=%d nh=%d nkv=%d D=%d", B, S, nh, nkv, D);
+    FLH_REQUIRE(cur >= 0 && cur + S <= T, FLH_B200_EINVAL, "positions %d .. %d do not fit a cache of %d", cur, cur + S - 1, T);
+    if (B == 0 || S == 0) return 0;
+    FLH_REQUIRE(qkv && cos && sin && q_out && k_cache && v_cache, FLH_B200_EINVAL, "null pointer");
+    FLH_REQUIRE(aligned16(qkv) && aligned16(cos) && aligned16(sin) && aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache),
+                FLH_B200_EALIGN, "pointers must be 16-byte aligned");
+    return launch_rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, D, T, cur, q_by_token, static_cast<cudaStream_t>(stream));
+}
 
 extern "C" {
 
@@ -223,13 +234,12 @@ int flh_b200_silu_mul_quant_token_asym_i4(const void *gu, int in_dtype, long M, 
 
 int flh_b200_rope_kv_f16(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
                          int B, int S, int nh, int nkv, int D, int T, int cur, void *stream) {
-    FLH_REQUIRE(B >= 0 && S >= 0 && nh > 0 && nkv > 0 && D > 0 && D % 8 == 0, FLH_B200_EINVAL, "bad shape B=%d S=%d nh=%d nkv=%d D=%d", B, S, nh, nkv, D);
-    FLH_REQUIRE(cur >= 0 && cur + S <= T, FLH_B200_EINVAL, "positions %d .. %d do not fit a cache of %d", cur, cur + S - 1, T);
-    if (B == 0 || S == 0) return 0;
-    FLH_REQUIRE(qkv && cos && sin && q_out && k_cache && v_cache, FLH_B200_EINVAL, "null pointer");
-    FLH_REQUIRE(aligned16(qkv) && aligned16(cos) && aligned16(sin) && aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache),
-                FLH_B200_EALIGN, "pointers must be 16-byte aligned");
-    return launch_rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, D, T, cur, static_cast<cudaStream_t>(stream));
+    return rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, D, T, cur, 0, stream);
+}
+
+int flh_b200_rope_kv_by_token_f16(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
+                                  int B, int S, int nh, int nkv, int D, int T, int cur, void *stream) {
+    return rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, D, T, cur, 1, stream);
 }
 
 const char *flh_b200_quant_token_kernel(long M, long K, int hadamard, int kfac) {

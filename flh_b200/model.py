@@ -169,8 +169,10 @@ class DecoderLayer(torch.nn.Module):
                 else:
                     kc = torch.empty((B, self.nkv, S, hd), dtype=qkv.dtype, device=qkv.device)
                     vc = torch.empty_like(kc)
-                qh = torch.empty((B, self.nh, S, hd), dtype=qkv.dtype, device=qkv.device)
-                _CUDA.rope_kv(qkv.view(B * S, -1), tables[0], tables[1], qh, kc, vc, B, S, self.nh, self.nkv, cur)
+                # q stays in token order: the attention output follows its layout and needs no transposing copy
+                qh = torch.empty((B, S, self.nh, hd), dtype=qkv.dtype, device=qkv.device)
+                _CUDA.rope_kv(qkv.view(B * S, -1), tables[0], tables[1], qh, kc, vc, B, S, self.nh, self.nkv, cur, q_by_token=True)
+                qh = qh.transpose(1, 2)
                 kh, vh = kc[:, :, :cur + S], vc[:, :, :cur + S]
             else:
                 qh, kh, vh = qkv.split((self.nh * hd, self.nkv * hd, self.nkv * hd), dim=-1)
@@ -288,5 +290,5 @@ class Decoder(torch.nn.Module):
             x, pre = out if isinstance(out, tuple) else (out, None)
         if sp:
             x = gather_rows(x, None, blocks).view(B, S, -1)
-        x = self.norm(x)
-        return x if self.head is None else self.head(x[:, -1:])
+        # the head reads the last position only: the others need no final norm
+        return self.norm(x) if self.head is None else self.head(self.norm(x[:, -1:]))

@@ -161,6 +161,10 @@ int flh_b200_silu_mul_quant_token_asym_i4(const void *gu, int in_dtype, long M, 
  * D % 8 == 0, cur + S <= T.  The reference does this as split, rotary, transpose and cache update (modeling_llama.py:396-440). */
 int flh_b200_rope_kv_f16(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
                          int B, int S, int nh, int nkv, int D, int T, int cur, void *stream);
+/* The same with q_out as [B, S, nh, D]: an attention call that is given that tensor transposed leaves its output in the same
+ * order, which is the row order the next linear reads. */
+int flh_b200_rope_kv_by_token_f16(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
+                                  int B, int S, int nh, int nkv, int D, int T, int cur, void *stream);
 
 /* HOST helpers: build the factor table of a kfac x kfac matrix of +1/-1 (int8, row-major, host
  * memory).  Layout: bit rows out[k * words + w], bit b = 1 when signs[k][32 w + b] < 0,

@@ -101,3 +101,38 @@ def test_ring_with_group_scales(cuda, m, n, k, mode):
     ref = O.gemm_i4_dequant(ap, bp, sa, sb).astype(np.float64)
     err = np.abs(d1.cpu().numpy().astype(np.float64) - ref)
     assert (err <= bound + 2.0 ** -10 * np.abs(ref) + 2.0 ** -24).all(), err.max()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_silu_of_every_gate(cuda, bf16):
+    """SiLU rounds a function of one 16-bit value: all 65,536 of them (but NaN), beside two values of up."""
+    bits = np.arange(65536, dtype=np.uint16)
+    g = O.bf16_bits_to_f32(bits) if bf16 else bits.view(np.float16).astype(np.float32)
+    bits = bits[~np.isnan(g)]
+    bits = np.concatenate([bits, bits[:(-len(bits)) % 64]])
+    up = (O.f32_to_bf16_bits(np.array([1.0, -2.75], np.float32)) if bf16 else np.array([1.0, -2.75], np.float16)).view(np.uint16)
+    gu = np.stack([np.concatenate([bits, np.full_like(bits, u)]) for u in up])
+    x = torch.from_numpy(gu.view(np.int16)).cuda().view(torch.bfloat16 if bf16 else torch.float16)
+    want = O.silu_mul16(gu if bf16 else gu.view(np.float16), bf16=bf16)
+    got = cuda.silu_mul(x).view(torch.int16).cpu().numpy().view(np.uint16)
+    assert np.array_equal(got, want.view(np.uint16))
+
+
+@pytest.mark.parametrize("D,B,S", [(128, 2, 40), (128, 3, 1), (40, 1, 700), (8, 2, 3)])
+def test_rope_by_token_is_the_transposed_form(cuda, D, B, S):
+    nh, nkv, cur, T = 6, 2, 3, S + 5
+    g = torch.Generator(device="cuda").manual_seed(3)
+    qkv = torch.randn(B * S, (nh + 2 * nkv) * D, device="cuda", generator=g).half()
+    ang = torch.randn(S, D // 2, device="cuda", generator=g)
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    outs = []
+    for by_token in (False, True):
+        kc, vc = torch.zeros(B, nkv, T, D, device="cuda").half(), torch.zeros(B, nkv, T, D, device="cuda").half()
+        q = torch.empty((B, S, nh, D) if by_token else (B, nh, S, D), dtype=torch.float16, device="cuda")
+        cuda.rope_kv(qkv, cos, sin, q, kc, vc, B, S, nh, nkv, cur, q_by_token=by_token)
+        outs.append((q.transpose(1, 2) if by_token else q, kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    x = qkv.view(B, S, nh + 2 * nkv, D)[:, :, :nh].float()
+    c, s = cos[None, :, None], sin[None, :, None]
+    want = torch.cat((x[..., :D // 2] * c - x[..., D // 2:] * s, x[..., D // 2:] * c + x[..., :D // 2] * s), -1).half()
+    assert torch.equal(outs[0][0], want.transpose(1, 2))
