@@ -136,3 +136,16 @@ def test_rope_by_token_is_the_transposed_form(cuda, D, B, S):
     c, s = cos[None, :, None], sin[None, :, None]
     want = torch.cat((x[..., :D // 2] * c - x[..., D // 2:] * s, x[..., D // 2:] * c + x[..., :D // 2] * s), -1).half()
     assert torch.equal(outs[0][0], want.transpose(1, 2))
+
+
+@pytest.mark.parametrize("m,k", [(1, 8), (3, 2056), (16, 4096), (33, 8192)])
+def test_rmsnorm(cuda, m, k):
+    """Binary32 sums in another order and a correctly rounded 1 / sqrt: one ulp of each of the two float16 roundings (2^-10 each)."""
+    from flh_b200.model import RMSNorm
+    x = torch.from_numpy(rs(m + k).standard_normal((m, k + 8)).astype(np.float16)).cuda()[:, :k]
+    norm = RMSNorm(k, 1e-5).cuda()
+    norm.weight.data.copy_(torch.from_numpy(rs(5).uniform(0.5, 2.0, k).astype(np.float16)))
+    v = x.double()
+    want = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5) * norm.weight.double()
+    err = (norm(x).double() - want).abs()
+    assert bool((err <= 2.0 ** -9 * want.abs() + 2.0 ** -24).all()), err.max().item()
