@@ -10,7 +10,9 @@ PyTorch is used only for device memory, streams and the device guard.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import functools
 import math
 
 import numpy as np
@@ -29,17 +31,23 @@ def _check(cond: bool, msg: str) -> None:
         raise RuntimeError(msg)
 
 
+# A call of this package is two or three launches, and the Python around them is what the smallest calls cost: 60-75 us a
+# linear before these helpers stopped making stream, guard and pointer objects and views that the call does not need.
+_getrawstream = getattr(torch._C, "_cuda_getCurrentRawStream", None)      # absent from CPU-only builds of torch
+_HERE = contextlib.nullcontext()
+
+
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _getrawstream(t.device.index)
 
 
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _guard(device):
     """Device guard around a C-ABI call (the library launches on the current device)."""
-    return torch.cuda.device(device)
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 # --------------------------------------------------------------------------- the nine pybind names
@@ -96,10 +104,31 @@ def _quant_group(x, gs, hadamard):
     rows = x.shape[0]
     q = torch.empty((rows, gs // 2), dtype=torch.uint8, device=x.device)
     s = torch.empty((rows,), dtype=torch.float16, device=x.device)
+    _launch_quant_group(x, rows, gs, hadamard, q, s)
+    return [q, s]
+
+
+def _launch_quant_group(x, rows, gs, hadamard, q, s):
     with _guard(x.device):
         _lib.check(_lib.load().flh_b200_quant_group_sym_i4(_ptr(x), rows, gs, int(hadamard), _ptr(q), _ptr(s), _stream(x)),
                    "quant_group_sym_i4")
-    return [q, s]
+
+
+def act_quant_group(x, gs: int, hadamard: bool):
+    """The group quantiser over the last dimension of x [.., K]: -> (q u8[.., K/2], scale f16[.., K/gs]), the scales those of the
+    normalised transform (the kernel's is un-normalised)."""
+    lead, K = x.shape[:-1], x.shape[-1]
+    _check(gs in (32, 64, 128), "group_size must be 32, 64, or 128")
+    _check(K % gs == 0, "the last dimension must be a multiple of group_size")
+    if not x.is_contiguous():
+        x = x.reshape(-1, gs)
+    _check(x.is_cuda, "Input tensor must be on CUDA")
+    _check(x.dtype == torch.float16, "Input tensor must be float16 (half)")
+    _check(x.is_contiguous(), "Input tensor must be contiguous")
+    q = torch.empty(lead + (K // 2,), dtype=torch.uint8, device=x.device)
+    s = torch.empty(lead + (K // gs,), dtype=torch.float16, device=x.device)
+    _launch_quant_group(x, x.numel() // gs, gs, hadamard, q, s)
+    return q, s / math.sqrt(gs) if hadamard else s
 
 
 def hadamard_and_quantize_i4(x):
@@ -152,7 +181,7 @@ _SIGN_CACHE: dict = {}
 
 def _sign_bits(n: int, device):
     """(kfac, device uint32 bit rows or None) for width n, cached per (width, device)."""
-    key = (n, str(device))
+    key = (n, device)
     hit = _SIGN_CACHE.get(key)
     if hit is not None:
         return hit
@@ -160,7 +189,7 @@ def _sign_bits(n: int, device):
     if k == 1:
         _SIGN_CACHE[key] = (1, None)
         return _SIGN_CACHE[key]
-    tkey = ("table", k, str(device))
+    tkey = ("table", k, device)
     if tkey not in _SIGN_CACHE:
         s8 = np.ascontiguousarray(signs, dtype=np.int8)
         out = np.zeros((_lib.load().flh_b200_sign_table_bytes(k) + 3) // 4, dtype=np.uint32)
@@ -185,7 +214,6 @@ def quant_token_asym_i4(x, hadamard: bool = True, clip: float = 1.0, exact: bool
     _check(x.dtype in (torch.float16, torch.bfloat16), "Input tensor must be float16 or bfloat16")
     _check(x.dim() == 2 and x.stride(1) == 1, "Input tensor must be 2D with unit inner stride")
     M, K = x.shape
-    kfac, bits = _sign_bits(K, x.device) if hadamard else (1, None)
     if out is not None:
         q, s, z = out
         _check(q.dtype == torch.uint8 and q.is_contiguous() and q.numel() == M * (K // 2) and q.device == x.device, "out[0] must be contiguous uint8 [M, K/2]")
@@ -195,11 +223,31 @@ def quant_token_asym_i4(x, hadamard: bool = True, clip: float = 1.0, exact: bool
         q = torch.empty((M, K // 2), dtype=torch.uint8, device=x.device)
         s = torch.empty((M,), dtype=torch.float16, device=x.device)
         z = torch.empty((M,), dtype=torch.float16, device=x.device)
+    _launch_quant_token(x, M, K, x.stride(0) if M > 1 else K, hadamard, clip, exact, q, s, z)
+    return q, s, z
+
+
+def _launch_quant_token(x, M, K, ld, hadamard, clip, exact, q, s, z):
+    kfac, bits = _sign_bits(K, x.device) if hadamard else (1, None)
     with _guard(x.device):
         _lib.check(_lib.load().flh_b200_quant_token_asym_i4(
-            _ptr(x), BF16 if x.dtype == torch.bfloat16 else F16, M, K, x.stride(0) if M > 1 else K,
+            _ptr(x), BF16 if x.dtype == torch.bfloat16 else F16, M, K, ld,
             (2 if exact else 1) if hadamard else 0, kfac,
             _ptr(bits), float(clip), _ptr(q), _ptr(s), _ptr(z), _stream(x)), "quant_token_asym_i4")
+
+
+def act_quant_token(x, hadamard: bool, clip: float):
+    """quant_token_asym_i4 over the last dimension of x [.., K]: -> (q u8[.., K/2], scale f16[.., 1], zero f16[.., 1])."""
+    lead, K = x.shape[:-1], x.shape[-1]
+    if not x.is_contiguous() or x.numel() == 0:
+        q, s, z = quant_token_asym_i4(x.reshape(-1, K), hadamard=hadamard, clip=clip)
+        return q.view(lead + (K // 2,)), s.view(lead + (1,)), z.view(lead + (1,))
+    _check(x.is_cuda, "Input tensor must be on CUDA")
+    _check(x.dtype in (torch.float16, torch.bfloat16), "Input tensor must be float16 or bfloat16")
+    q = torch.empty(lead + (K // 2,), dtype=torch.uint8, device=x.device)
+    s = torch.empty(lead + (1,), dtype=torch.float16, device=x.device)
+    z = torch.empty(lead + (1,), dtype=torch.float16, device=x.device)
+    _launch_quant_token(x, x.numel() // K, K, K, hadamard, clip, False, q, s, z)
     return q, s, z
 
 
@@ -317,7 +365,7 @@ _WORKSPACES: dict = {}
 def _workspace(device, stream: int, nbytes: int):
     """Zero-initialised scratch for the split-K decode kernel, one per (device, stream): launches on one
     stream run in order, so they may share it; the kernel leaves its counters zeroed."""
-    key = (str(device), stream)
+    key = (device, stream)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 8 << 20), dtype=torch.uint8, device=device)
@@ -334,7 +382,7 @@ def _scratch(device, stream: int, nbytes: int):
     of the graph's own instead: the shared buffer is replaced when a larger call comes, the graph would go on using it."""
     if torch.cuda.is_current_stream_capturing():
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    key = (str(device), stream)
+    key = (device, stream)
     ws = _SCRATCH.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
@@ -349,30 +397,42 @@ def gemm_i4_dequant(A, B, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=Non
     M, Kp = A.shape
     N = B.shape[0]
     K = Kp * 2
-    A_scale = A_scale.reshape(M, -1)
-    B_scale = B_scale.reshape(N, -1)
+    if A_scale.dim() != 2 or A_scale.shape[0] != M or M == 0:
+        A_scale = A_scale.reshape(M, -1)
+    if B_scale.dim() != 2 or B_scale.shape[0] != N or N == 0:
+        B_scale = B_scale.reshape(N, -1)
     _check(A_scale.shape[1] > 0 and K % A_scale.shape[1] == 0, "A_scale columns must divide K")
     _check(B_scale.shape[1] > 0 and K % B_scale.shape[1] == 0, "B_scale columns must divide K")
-    ag, bg = K // A_scale.shape[1], K // B_scale.shape[1]
     D = out if out is not None else torch.empty((M, N), dtype=out_dtype, device=A.device)
+    _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, K // A_scale.shape[1], K // B_scale.shape[1], algo)
+    return D
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_plan(lib, M, N, K, ag, bg, algo, has_zero):
+    """(workspace bytes, whether it must be zeroed) of a GEMM: a function of the sizes alone."""
+    # what AUTO can use depends on the zero-points only where there are group scales: those keep the kernels without workspace of that kind
+    auto = algo == GEMM_AUTO and not (has_zero and min(ag, bg) < K)
+    need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if auto else algo)
+    resolved = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
+    return need, M <= 64 and resolved not in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_GROUP_F8)
+
+
+def _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, ag, bg, algo):
     lib = _lib.load()
     with _guard(A.device):
         stream = _stream(A)
-        # what AUTO can use depends on the zero-points only where there are group scales: those keep the kernels without workspace of that kind
-        auto = algo == GEMM_AUTO and not (A_zero is not None and min(ag, bg) < K)
-        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if auto else algo)
-        resolved = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
+        need, zeroed = _gemm_plan(lib, M, N, K, ag, bg, algo, A_zero is not None)
         if not need:
             ws = None
-        elif M > 64 or resolved in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_GROUP_F8):
-            ws = _scratch(A.device, stream, need)          # expanded operands: any contents
-        else:
+        elif zeroed:
             ws = _workspace(A.device, stream, need)        # split-K: zeroed counters, left zeroed
+        else:
+            ws = _scratch(A.device, stream, need)          # expanded operands: any contents
         _lib.check(lib.flh_b200_gemm_i4_dequant(
             _ptr(A), _ptr(B), _ptr(A_scale), _ptr(A_zero), _ptr(B_scale), _ptr(B_rowsum), _ptr(bias), _ptr(D),
             M, N, K, ag, bg, BF16 if D.dtype == torch.bfloat16 else F16, algo, _ptr(ws), ws.numel() if ws is not None else 0,
             stream), "gemm_i4_dequant")
-    return D
 
 
 def expand_i4(B):

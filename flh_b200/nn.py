@@ -42,18 +42,11 @@ class ActQuantizer(torch.nn.Module):
 
     def forward(self, x):
         """Returns (scale, zero_point or None, packed uint8 codes), as flh/nn/quantization.py:156-162."""
-        lead, K = x.shape[:-1], x.shape[-1]
         if self.sym:
-            gs = self.group_size if self.group_size and self.group_size > 0 else 128
-            xg = x.reshape(-1, gs)
-            if self.use_hadamard:
-                q, scales = _CUDA.hadamard_and_quantize_i4_gs(xg, gs)
-                scales = scales / math.sqrt(gs)          # the kernel's transform is un-normalised
-            else:
-                q, scales = _CUDA.quant_and_pack_i4_gs(xg, gs)
-            return scales.view(lead + (K // gs,)), None, q.view(lead + (K // 2,))
-        q, s, z = _CUDA.quant_token_asym_i4(x.reshape(-1, K), hadamard=self.use_hadamard, clip=self.input_clip_ratio)
-        return s.view(lead + (1,)), z.view(lead + (1,)), q.view(lead + (K // 2,))
+            q, s = _CUDA.act_quant_group(x, self.group_size if self.group_size and self.group_size > 0 else 128, self.use_hadamard)
+            return s, None, q
+        q, s, z = _CUDA.act_quant_token(x, self.use_hadamard, self.input_clip_ratio)
+        return s, z, q
 
     def forward_origin(self, x):
         """PyTorch twin of forward (flh/nn/quantization.py:163-241): float64 transform, then the
@@ -268,20 +261,24 @@ class LinearFLH(torch.nn.Module):
         contiguous [M, N] tensor to write into instead of allocating."""
         lead = x.shape[:-1]
         M = x.numel() // x.shape[-1]
-        a_scale = a_scale.reshape(M, -1)
-        ga, gb = self.in_features // a_scale.shape[1], self.in_features // self.w_scale.shape[1]
+        N, w_scale = self.out_features, self.w_scale
+        if M == 0 or a_scale.dim() != 2 or a_scale.shape[0] != M or not a_scale.is_contiguous():
+            a_scale = a_scale.reshape(M, -1)
+        ga, gb = self.in_features // a_scale.shape[1], self.in_features // w_scale.shape[1]
         rs = None
         if a_zero is not None:
-            a_zero = a_zero.reshape(M, -1)
+            if not a_zero.is_contiguous():
+                a_zero = a_zero.reshape(M, -1)
             rs = self.w_rowsum(min(ga, gb))
+        if x.dim() != 2 or M == 0:
+            x = x.reshape(M, -1)
+        dtype = out_dtype or w_scale.dtype
         if self._w_i8 is not None and a_scale.shape[1] == 1 and M >= self.PREPACK_MIN_ROWS:
-            y = _CUDA.gemm_i8w_dequant(x.reshape(M, -1), self._w_i8, a_scale, self.w_scale, A_zero=a_zero, B_rowsum=rs,
-                                       bias=self.bias, out_dtype=out_dtype or self.w_scale.dtype, out=out)
+            y = _CUDA.gemm_i8w_dequant(x, self._w_i8, a_scale, w_scale, A_zero=a_zero, B_rowsum=rs, bias=self.bias, out_dtype=dtype, out=out)
         else:
-            y = _CUDA.gemm_i4_dequant(x.reshape(M, -1), self.w_packed.view(self.out_features, self.in_features // 2),
-                                      a_scale, self.w_scale, A_zero=a_zero, B_rowsum=rs, bias=self.bias,
-                                      out_dtype=out_dtype or self.w_scale.dtype, out=out)
-        return y.view(lead + (self.out_features,))
+            y = _CUDA.gemm_i4_dequant(x, self.w_packed.view(N, self.in_features // 2), a_scale, w_scale, A_zero=a_zero, B_rowsum=rs,
+                                      bias=self.bias, out_dtype=dtype, out=out)
+        return y if y.shape == lead + (N,) else y.view(lead + (N,))
 
     def forward_torch(self, x, a_scale=None, a_zero=None, x_is_packed=True, is_symmetric=None):
         """PyTorch twin (flh/nn/linear.py:134-152): unpack, (q - zero) * scale, F.linear."""

@@ -149,3 +149,27 @@ def test_rmsnorm(cuda, m, k):
     want = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5) * norm.weight.double()
     err = (norm(x).double() - want).abs()
     assert bool((err <= 2.0 ** -9 * want.abs() + 2.0 ** -24).all()), err.max().item()
+
+
+@pytest.mark.parametrize("shape", [(128,), (3, 256), (2, 5, 384)])
+@pytest.mark.parametrize("kind", ["group", "group_had", "token"])
+def test_quantiser_module_shapes_and_strides(cuda, shape, kind):
+    """The module's outputs follow the input's leading dimensions, contiguous or not, as the functions on matrices give them."""
+    from flh_b200.nn import ActQuantizer
+    sym, had = kind != "token", kind == "group_had"
+    quant = ActQuantizer(bits=4, group_size=128 if sym else -1, sym=sym, use_hadamard=had, packed_output=True)
+    K = shape[-1]
+    base = torch.randn(shape[:-1] + (K + 64,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).half()
+    for x in (base[..., :K].contiguous(), base[..., :K]):
+        s, z, q = quant(x)
+        flat = x.reshape(-1, K).contiguous()
+        if sym:
+            q0, s0 = (cuda.hadamard_and_quantize_i4 if had else cuda.quant_and_pack_i4)(flat.view(-1, 128))
+            s0 = s0 / 128 ** 0.5 if had else s0
+            assert z is None and s.shape == shape[:-1] + (K // 128,)
+        else:
+            q0, s0, z0 = cuda.quant_token_asym_i4(flat, hadamard=False)
+            assert s.shape == z.shape == shape[:-1] + (1,) and torch.equal(z.reshape(-1), z0)
+        assert q.shape == shape[:-1] + (K // 2,) and torch.equal(q.reshape(-1), q0.reshape(-1)) and torch.equal(s.reshape(-1), s0.reshape(-1))
+    with pytest.raises(RuntimeError):
+        ActQuantizer(bits=4, group_size=128, sym=True, use_hadamard=False, packed_output=True)(torch.zeros(2, 192, device="cuda").half())
