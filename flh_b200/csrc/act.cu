@@ -15,6 +15,8 @@ constexpr int kSiluThreads = 128;
 template <bool BF16>
 __global__ void __launch_bounds__(kSiluThreads) silu_mul_kernel(const uint8_t *__restrict__ gu, long M, long F, long ld_bytes, uint8_t *__restrict__ out) {
     const long c = (long)blockIdx.x * kSiluThreads + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (c >= F / 8) return;
     const long step = gridDim.y;
     for (long m = blockIdx.y; m < M; m += 2 * step) {
@@ -33,6 +35,8 @@ constexpr int kNormThreads = 256, kNormPieces = 4;             // rows of up to 
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const uint4 *__restrict__ x, const uint4 *__restrict__ w, int pieces, long ld16,
                                                                float eps, float inv_n, uint4 *__restrict__ out) {
     __shared__ float part[kNormThreads / 32];
+    pdl_wait();
+    pdl_trigger();
     const uint4 *row = x + blockIdx.x * ld16;
     uint4 v[kNormPieces];
     float ssq = 0.0f;
@@ -93,6 +97,8 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(const RopeParams p) {
     const int half = p.D / 2, vec = half / W;                      // pieces of W elements per half head
     const int heads = p.nh + 2 * p.nkv, items = heads * vec;
     const long token = blockIdx.x;
+    pdl_wait();
+    pdl_trigger();
     const int b = (int)(token / p.S), s = (int)(token - (long)b * p.S);
     for (int i = blockIdx.y * 256 + threadIdx.x; i < items; i += gridDim.y * 256) {
         const int h = i / vec, v = i - h * vec;
@@ -145,16 +151,13 @@ int launch_silu_mul(const void *gu, int in_dtype, long M, long F, long ld, void 
     if (rows > M) rows = M;
     const dim3 grid((unsigned)cols, (unsigned)rows);
     if (in_dtype == FLH_B200_BF16)
-        silu_mul_kernel<true><<<grid, kSiluThreads, 0, stream>>>(static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out));
-    else
-        silu_mul_kernel<false><<<grid, kSiluThreads, 0, stream>>>(static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out));
-    return cuda_status(cudaGetLastError(), "silu_mul launch");
+        return cuda_status(launch_pdl(silu_mul_kernel<true>, grid, kSiluThreads, 0, stream, static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out)), "silu_mul launch");
+    return cuda_status(launch_pdl(silu_mul_kernel<false>, grid, kSiluThreads, 0, stream, static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out)), "silu_mul launch");
 }
 
 int launch_rmsnorm(const void *x, const void *w, long M, long K, long ld, float eps, void *out, cudaStream_t stream) {
-    rmsnorm_kernel<<<(unsigned)M, kNormThreads, 0, stream>>>(static_cast<const uint4 *>(x), static_cast<const uint4 *>(w), (int)(K / 8), ld / 8,
-                                                             eps, 1.0f / (float)K, static_cast<uint4 *>(out));
-    return cuda_status(cudaGetLastError(), "rmsnorm launch");
+    return cuda_status(launch_pdl(rmsnorm_kernel, dim3((unsigned)M), kNormThreads, 0, stream, static_cast<const uint4 *>(x), static_cast<const uint4 *>(w),
+                                  (int)(K / 8), ld / 8, eps, 1.0f / (float)K, static_cast<uint4 *>(out)), "rmsnorm launch");
 }
 
 int launch_rope_kv(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,
@@ -172,9 +175,7 @@ int launch_rope_kv(const void *qkv, const float *cos, const float *sin, void *q_
     const long items = (long)(nh + 2 * nkv) * (D / 2 / w), parts = (items + 255) / 256;
     // a token's heads are spread over several blocks only while the tokens alone do not fill the GPU
     const dim3 grid((unsigned)tokens, (unsigned)(tokens >= 4L * kNumSMs ? 1 : parts));
-    if (w == 8) rope_kv_kernel<8><<<grid, 256, 0, stream>>>(p);
-    else rope_kv_kernel<4><<<grid, 256, 0, stream>>>(p);
-    return cuda_status(cudaGetLastError(), "rope_kv launch");
+    return cuda_status(launch_pdl(w == 8 ? rope_kv_kernel<8> : rope_kv_kernel<4>, grid, 256, 0, stream, p), "rope_kv launch");
 }
 
 }  // namespace flh

@@ -30,6 +30,25 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may start while the one before it on the stream still runs
+// (once every CTA of that one has called pdl_trigger or left).  The rules that keep it safe:
+//   * nothing that an earlier kernel wrote is read, and nothing is written, before pdl_wait — which returns when the kernel
+//     before has completed, and with it, because it waited too, everything before that;
+//   * pdl_trigger comes after pdl_wait (or in a kernel launched normally), and in a kernel that uses tensor memory after its
+//     allocation: a dependent that allocates must never stand in front of the kernel it waits for.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Packed binary32 pairs (sm_100): two IEEE adds / fused multiply-adds per instruction.
 // Written as plain integer arithmetic (not an opaque asm mov) so that the compiler can keep the two
 // halves in an aligned register pair without moving them.

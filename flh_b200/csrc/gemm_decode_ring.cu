@@ -108,6 +108,7 @@ gemm_decode_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     }
     if (!GROUPED && tid >= 64 && tid < 64 + TOK) {
         const int j = tid - 64;
+        pdl_wait();
         sa_s[j] = j < p.M ? __half2float(p.a_scale[j]) : 0.0f;
         za_s[j] = ZERO && j < p.M ? (int)__half2float(p.a_zero[j]) : 0;
     }
@@ -118,6 +119,13 @@ gemm_decode_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         if (lane == 0) {
             int it = 0;
             bool ok = true;
+            // while the kernel that makes the tokens still runs, the first stages of weights come into the L2 cache (a prefetch
+            // reads no value, so it needs no order with whatever wrote them)
+            for (int st = 0; st < S && st < p.steps && (int)blockIdx.x < p.tiles; ++st)
+#pragma unroll
+                for (int k = 0; k < WK; ++k) tma_prefetch_2d(&map_w, (st * WK + k) * 128, blockIdx.x * BR);
+            pdl_wait();
+            pdl_trigger();
             for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
                 for (int st = 0; st < p.steps; ++st, ++it) {
                     const int s = it % S;
@@ -139,6 +147,7 @@ gemm_decode_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         }
     } else {
         // ------------------------------------------------------------ consumers
+        pdl_wait();
         const int kg = warp % WK, wr = warp / WK;
         const int g = lane >> 2, t = lane & 3, rho = (g >> 1) | ((g & 1) << 2);
         const int frag = rho * 128 + ((t ^ rho) << 4);                // chunk t of row rho; chunk 4 + t is at ^ 64
@@ -296,8 +305,7 @@ int launch_ring(const CUtensorMap &mw, const CUtensorMap &mx, RingParams p, cuda
     p.steps = (p.chunks + WK - 1) / WK;
     p.tiles = p.N / Plan::BR;
     const int sms = tc_device_sms();
-    kern<<<p.tiles < sms ? p.tiles : sms, kThreadsRing, Plan::kBytes, stream>>>(mw, mx, p);
-    return cuda_status(cudaGetLastError(), "gemm_decode_ring launch");
+    return cuda_status(launch_pdl(kern, dim3(p.tiles < sms ? p.tiles : sms), kThreadsRing, Plan::kBytes, stream, mw, mx, p), "gemm_decode_ring launch");
 }
 
 // packed matrix of rows x K / 2 bytes; box = box_rows x 128 bytes with the 128-byte swizzle, zeros outside

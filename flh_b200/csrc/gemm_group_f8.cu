@@ -60,6 +60,7 @@ struct PrepParams {
 __global__ void __launch_bounds__(256) prep_group_f8_kernel(const PrepParams p) {
     const long stride = (long)gridDim.x * blockDim.x, t0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long total = p.a16 + p.b16;
+    pdl_trigger();
     constexpr int U = 4;                                 // loads in flight
     for (long i0 = t0; i0 < total; i0 += stride * U) {
         uint4 wv[U];
@@ -172,6 +173,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::);     // 128 x 72 + 256 x 216 = 384 x 168, what the block is launched with
         if (warp == 0 && lane == 0) {
             // -------------------------------------------------------- TMA producer (own halves)
+            pdl_wait();                      // the operands are made by the kernel before; the set-up above overlapped it
             int it = 0;
             bool ok = true;
             for (int tile = first; tile < p.num_tiles && ok; tile += step) {
@@ -220,6 +222,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
         } else if (warp == 2 && lane == 0) {
             // -------------------------------------------------------- scales of every block
+            pdl_wait();
             int it = 0;
             bool ok = true;
             for (int tile = first; tile < p.num_tiles && ok; tile += step) {
@@ -355,13 +358,15 @@ int launch_f8(const CUtensorMap &ma, const CUtensorMap &mb, F8Params p, cudaStre
     p.m_blocks = (p.M + 2 * BM - 1) / (2 * BM);
     p.num_tiles = p.m_blocks * (p.N / BN);
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cfg.blockDim = dim3(Plan::kThreads);
     cfg.dynamicSmemBytes = Plan::kBytes;
     cfg.stream = stream;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     // persistent: no more pairs than can be resident at once
     static int max_pairs = 0;
     if (max_pairs == 0) {

@@ -49,14 +49,25 @@ __device__ __forceinline__ void tc_mma_i8_plain(uint32_t d_tmem, uint64_t adesc,
 // ---- expansion --------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) expand_i4_kernel(const uint4 *__restrict__ in, uint4 *__restrict__ out, long n16) {
     const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride) {
-        const uint4 w = ldg_nc_v4(in + i);
+    pdl_trigger();
+    constexpr int U = 4;                                 // loads in flight
+    for (long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n16; i0 += stride * U) {
+        uint4 wv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * stride < n16) wv[u] = ldg_nc_v4(in + i0 + u * stride);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+        const long i = i0 + u * stride;
+        if (i >= n16) break;
+        const uint4 w = wv[u];
         uint4 e, o;
         e.x = (w.x << 4) & 0xF0F0F0F0u; e.y = (w.y << 4) & 0xF0F0F0F0u;
         e.z = (w.z << 4) & 0xF0F0F0F0u; e.w = (w.w << 4) & 0xF0F0F0F0u;
         o.x = w.x & 0xF0F0F0F0u; o.y = w.y & 0xF0F0F0F0u; o.z = w.z & 0xF0F0F0F0u; o.w = w.w & 0xF0F0F0F0u;
         out[2 * i] = e;
         out[2 * i + 1] = o;
+        }
     }
 }
 
@@ -134,6 +145,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (own halves)
         if (lane == 0) {
+            pdl_wait();                  // the operands are made by the kernel before; the set-up above overlapped it
             int it = 0;
             bool ok = true;
             unsigned long long w1 = 0;
@@ -267,14 +279,17 @@ int launch_i8(const CUtensorMap &ma, const CUtensorMap &mb, const I8Params &p, c
     q.num_tiles = q.m_blocks * (p.N / BN);
     const int sms = tc_device_sms();
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
     cfg.blockDim = dim3(Plan::kThreads);
     cfg.dynamicSmemBytes = Plan::kBytes;
     cfg.stream = stream;
     if (PAIR) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr; cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
         // the kernel is persistent: launch no more clusters than can be resident at once
         static int max_pairs = 0;
         if (max_pairs == 0) {

@@ -101,6 +101,8 @@ quant_group_sym_kernel(const uint4 *__restrict__ x, uint32_t *__restrict__ q,
     const long tid = (long)blockIdx.x * kThreads + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int lig = lane & (L - 1);
+    pdl_wait();
+    pdl_trigger();
 
     for (long c0 = tid; c0 - lane < total_chunks; c0 += nthreads * kUnroll) {
         uint4 v[kUnroll];
@@ -186,6 +188,8 @@ quant_group_thread_kernel(const uint8_t *__restrict__ x, uint4 *__restrict__ q, 
     const long tiles = (groups + 31) >> 5, total_chunks = groups * (GS / 8);
     const long nwarps = (long)gridDim.x * kTWarps;
     long tile = (long)blockIdx.x * kTWarps + warp;
+    pdl_wait();
+    pdl_trigger();
     if (tile < tiles) stage_groups<GS>(x, tile, total_chunks, stage, lane);
 
     for (; tile < tiles; tile += nwarps) {
@@ -332,22 +336,24 @@ int launch_quant_group_sym(const void *x, long rows, int gs, int hadamard, uint8
         const uint8_t *xb = static_cast<const uint8_t *>(x);
         uint4 *qo4 = reinterpret_cast<uint4 *>(q);
         __half *so4 = static_cast<__half *>(scales);
-#define FLH_TLAUNCH(GS_, H_) quant_group_thread_kernel<GS_, H_><<<(unsigned)grid, kTWarps * 32, kTWarps * 64 * GS_, stream>>>(xb, qo4, so4, rows)
+#define FLH_TLAUNCH(GS_, H_) e = launch_pdl(quant_group_thread_kernel<GS_, H_>, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * GS_, stream, xb, qo4, so4, rows, 0.0f)
+        cudaError_t e;
         if (gs == 128) { if (hadamard) FLH_TLAUNCH(128, true); else FLH_TLAUNCH(128, false); }
         else if (gs == 64) { if (hadamard) FLH_TLAUNCH(64, true); else FLH_TLAUNCH(64, false); }
         else { if (hadamard) FLH_TLAUNCH(32, true); else FLH_TLAUNCH(32, false); }
 #undef FLH_TLAUNCH
-        return cuda_status(cudaGetLastError(), "quant_group_thread launch");
+        return cuda_status(e, "quant_group_thread launch");
     }
     const uint4 *xi = static_cast<const uint4 *>(x);
     uint32_t *qo = reinterpret_cast<uint32_t *>(q);
     __half *so = static_cast<__half *>(scales);
-#define FLH_LAUNCH(LG, H) quant_group_sym_kernel<LG, H><<<grid_for(quant_group_sym_kernel<LG, H>, chunks), kThreads, 0, stream>>>(xi, qo, so, chunks)
+#define FLH_LAUNCH(LG, H) e = launch_pdl(quant_group_sym_kernel<LG, H>, dim3(grid_for(quant_group_sym_kernel<LG, H>, chunks)), kThreads, 0, stream, xi, qo, so, chunks)
+    cudaError_t e;
     if (gs == 128) { if (hadamard) FLH_LAUNCH(7, true); else FLH_LAUNCH(7, false); }
     else if (gs == 64) { if (hadamard) FLH_LAUNCH(6, true); else FLH_LAUNCH(6, false); }
     else { if (hadamard) FLH_LAUNCH(5, true); else FLH_LAUNCH(5, false); }
 #undef FLH_LAUNCH
-    return cuda_status(cudaGetLastError(), "quant_group_sym launch");
+    return cuda_status(e, "quant_group_sym launch");
 }
 
 // rows of 4096 halves: RMS-norm + group-128 (transform +) symmetric int4 + pack
@@ -359,9 +365,8 @@ int launch_rmsnorm_quant_group(const void *x, long M, int hadamard, float eps, u
     const uint8_t *xb = static_cast<const uint8_t *>(x);
     uint4 *qo4 = reinterpret_cast<uint4 *>(q);
     __half *so4 = static_cast<__half *>(scales);
-    if (hadamard) quant_group_thread_kernel<128, true, true><<<(unsigned)grid, kTWarps * 32, kTWarps * 64 * 128, stream>>>(xb, qo4, so4, groups, eps);
-    else quant_group_thread_kernel<128, false, true><<<(unsigned)grid, kTWarps * 32, kTWarps * 64 * 128, stream>>>(xb, qo4, so4, groups, eps);
-    return cuda_status(cudaGetLastError(), "rmsnorm_quant_group launch");
+    const auto kern = hadamard ? quant_group_thread_kernel<128, true, true> : quant_group_thread_kernel<128, false, true>;
+    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * 128, stream, xb, qo4, so4, groups, eps), "rmsnorm_quant_group launch");
 }
 
 int launch_fht_inplace(void *x, long rows, int n, cudaStream_t stream) {

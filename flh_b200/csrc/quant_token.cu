@@ -117,6 +117,8 @@ quant_token_asym_kernel(const TokenParams p) {
         __syncthreads();
     }
 
+    pdl_wait();
+    pdl_trigger();
     for (long row = blockIdx.x; row < p.M; row += gridDim.x) {
     float x[64];
 
@@ -473,8 +475,7 @@ int launch_one(const TokenParams &p, long M, cudaStream_t stream) {
     }
     TokenParams q = p;
     q.M = M;
-    kern<<<(unsigned)grid, threads, smem, stream>>>(q);
-    return cuda_status(cudaGetLastError(), "quant_token_asym launch");
+    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), threads, smem, stream, q), "quant_token_asym launch");
 }
 
 }  // namespace

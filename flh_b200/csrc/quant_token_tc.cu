@@ -154,6 +154,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) quant_token_tc_kernel(const __g
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();                              // all of the above (the sign operand above all) overlaps the kernel before
+    pdl_trigger();
     const long n_units = (p.M + R * NB - 1) / (R * NB);
     if (PROFILE && tid == 0) atomicAdd(&g_wait_tc[5], gtimer() - t_start);
     // a bounded wait, timed as a whole when profiling (try_wait may itself block for a while before it returns)
@@ -684,8 +686,7 @@ static int launch_tc(const void *x, const void *gu, int in_dtype, long M, long K
     }
     const long n_units = (M + (long)p.R * NB - 1) / ((long)p.R * NB);
     const long grid = n_units < kNumSMs ? n_units : kNumSMs;
-    kern<<<(unsigned)grid, kThreadsTc, smem, stream>>>(map, p);
-    return cuda_status(cudaGetLastError(), "quant_token_tc launch");
+    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), kThreadsTc, smem, stream, map, p), "quant_token_tc launch");
 }
 
 int launch_quant_token_tc(const void *x, int in_dtype, long M, long K, long ld, int kfac, const uint32_t *sign_bits,

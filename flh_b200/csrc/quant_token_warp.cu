@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm) quant_token_war
 
     const long nwarps = (long)gridDim.x * (kWarpsPerCta / W);    // rows in flight
     long row = (long)blockIdx.x * (kWarpsPerCta / W) + grp;
+    pdl_wait();
+    pdl_trigger();
     if (row < p.M) stage_row<W>(p, row, stage, t);
 
     for (; row < p.M; row += nwarps) {
@@ -349,8 +351,7 @@ int launch_quant_token_warp(const void *x, int in_dtype, long M, long K, long ld
     const int rows_per_cta = kWarpsPerCta / W;
     long grid = (M + rows_per_cta - 1) / rows_per_cta;
     if (grid > (long)kCtasPerSm * kNumSMs) grid = (long)kCtasPerSm * kNumSMs;
-    kern<<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
-    return cuda_status(cudaGetLastError(), "quant_token_warp launch");
+    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), kWarpsPerCta * 32, smem, stream, p), "quant_token_warp launch");
 }
 
 }  // namespace flh
