@@ -208,16 +208,18 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             for (int tile = first; tile < p.num_tiles && ok; tile += step) {
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % S, buf = it & 1;
-                    if (it >= 2 && !wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42)) { ok = false; break; }
+                    // the operands are there long before; the buffer is what this thread waits for, and what the epilogue waits for
+                    // is the first thing it commits
                     if (!wait_f8(full(s), (it / S) & 1, abort_flag, 43)) { ok = false; break; }
+                    if (it >= 2 && !wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = base + s * Plan::kStageBytes;
                     const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BM * BK);
 #pragma unroll
                     for (int k4 = 0; k4 < BK / 32; ++k4)
                         mma_f8_pair(tmem + buf * 256, adesc + 2 * k4, bdesc + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-                    tc_commit_pair(empty(s));
                     tc_commit_pair(acc_full(buf));
+                    tc_commit_pair(empty(s));
                 }
             }
         } else if (warp == 2 && lane == 0) {

@@ -36,7 +36,7 @@ def test_group_f8_extreme_codes(cuda, a, b):
 
 
 def test_group_f8_needs_its_workspace_and_auto_does_without(cuda):
-    lib, m, n, k = cuda._lib.load(), 300, 512, 1024
+    lib, m, n, k = cuda._lib.load(), 300, 512, 2048
     case = make_case(11, m, n, k, 128, 128, False)
     run_case(cuda, AUTO, case)
     A, B, SA, SB = (_dev(t) for t in case[:4])
@@ -45,6 +45,7 @@ def test_group_f8_needs_its_workspace_and_auto_does_without(cuda):
     call = lambda algo, ws, nbytes: lib.flh_b200_gemm_i4_dequant(A.data_ptr(), B.data_ptr(), SA.data_ptr(), None, SB.data_ptr(), None, None, D.data_ptr(),
                                                                  m, n, k, 128, 128, 0, algo, ws, nbytes, s)
     need = lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, F8)
+    assert need == lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, cuda.GEMM_AUTO_WORKSPACE)      # AUTO would take it
     ws = torch.empty(need, dtype=torch.uint8, device="cuda")
     assert call(F8, None, 0) != 0 and call(F8, ws.data_ptr(), need - 1) != 0
     want = O.gemm_i4_dequant(*case[:4]).view(np.uint16)
@@ -56,7 +57,7 @@ def test_group_f8_needs_its_workspace_and_auto_does_without(cuda):
 
 def test_group_f8_scratch_of_a_captured_call_outlives_a_larger_call(cuda):
     """A recorded launch keeps its own scratch: a later, larger call on the same stream must not take it away."""
-    small, large = make_case(21, 300, 512, 1024, 128, 128, False), make_case(22, 600, 1024, 2048, 128, 128, False)
+    small, large = make_case(21, 300, 512, 2048, 128, 128, False), make_case(22, 600, 1024, 4096, 128, 128, False)
     t = [_dev(x) for x in small[:4]]
     side = torch.cuda.Stream()
     with torch.cuda.stream(side):
