@@ -142,6 +142,7 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();                                     // the set-up overlaps the kernel that makes the tokens
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -503,8 +504,7 @@ int launch_t(const CUtensorMap &mw, const CUtensorMap &mx, const DecParams &p, i
     if (smem > 227 * 1024) return fail(FLH_B200_EUNSUPPORTED, "K = %d needs %d bytes of shared memory for the token scales", p.K, smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_status(e, "gemm_decode_tc attribute");
-    kern<<<grid, Plan::kThreads, smem, stream>>>(mw, mx, p);
-    return cuda_status(cudaGetLastError(), "gemm_decode_tc launch");
+    return cuda_status(launch_pdl(kern, dim3(grid), Plan::kThreads, smem, stream, mw, mx, p), "gemm_decode_tc launch");
 }
 
 template <int TOK>

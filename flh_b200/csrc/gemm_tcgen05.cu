@@ -139,6 +139,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();                              // the set-up overlaps the kernel that makes the activations
 
     if (tid < kNonEpiThreads) {
         if (GROUPED) {
@@ -537,8 +538,7 @@ int launch_t(const CUtensorMap &ma, const CUtensorMap &mb, const TcParams &p, cu
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = kNumSMs;
     }
     const int grid = q.num_tiles < sms ? q.num_tiles : sms;        // one persistent CTA per SM
-    kern<<<grid, Roles<GROUPED>::kNonEpi + Roles<GROUPED>::epi_threads(BN), smem, stream>>>(ma, mb, q);
-    return cuda_status(cudaGetLastError(), "gemm_tcgen05 launch");
+    return cuda_status(launch_pdl(kern, dim3(grid), Roles<GROUPED>::kNonEpi + Roles<GROUPED>::epi_threads(BN), smem, stream, ma, mb, q), "gemm_tcgen05 launch");
 }
 
 }  // namespace
