@@ -28,7 +28,7 @@ __device__ __forceinline__ float exp32(float t) {
 }
 
 // The same values for two gates at once in packed binary32, for finite gates of magnitude 2^-90 and up and, in bfloat16, above
-// -80 (silu2_takes; float16 has no smaller ones, and its quotients below -80 round to -0 either way).  There no step of exp32
+// -80 (silu_mul_8 looks; float16 has no smaller ones, and its quotients below -80 round to -0 either way).  There no step of exp32
 // rounds to a subnormal or overflows:
 //   * rint by adding 1.5 * 2^23, whose low bits then are n for the exponent;
 //   * the quotient by Newton-Raphson on a reciprocal estimate and a final fused residual step (Markstein, IBM J. Res. Dev. 34,
@@ -67,12 +67,6 @@ __device__ __forceinline__ uint64_t silu2(uint64_t g) {
     const uint64_t a = mul2(g, q);
     return fma2(fma2(nd, a, g), q, a);
 }
-template <bool BF16>
-__device__ __forceinline__ bool silu2_takes(float g) {
-    const float m = fabsf(g);
-    return m > (BF16 ? 8.0e-28f : 0.0f) && m < 3.0e38f && (!BF16 || g > -80.0f);
-}
-
 // two neighbouring elements at once: g2, u2 hold two 16-bit values each (low half = the lower index)
 template <bool BF16>
 __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g2, uint32_t u2) {
@@ -85,13 +79,8 @@ __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g2, uint32_t u2) {
         const float2 uf = __half22float2(*reinterpret_cast<const __half2 *>(&u2));
         g0 = gf.x; g1 = gf.y; u0 = uf.x; u1 = uf.y;
     }
-    float s0, s1;
-    if (silu2_takes<BF16>(g0) && silu2_takes<BF16>(g1)) {
-        unpack2(silu2(pack2(g0, g1)), s0, s1);
-    } else {
-        s0 = __fdiv_rn(g0, __fadd_rn(1.0f, exp32(-g0)));
-        s1 = __fdiv_rn(g1, __fadd_rn(1.0f, exp32(-g1)));
-    }
+    const float s0 = __fdiv_rn(g0, __fadd_rn(1.0f, exp32(-g0)));
+    const float s1 = __fdiv_rn(g1, __fadd_rn(1.0f, exp32(-g1)));
     if (BF16) {
         const float a0 = __bfloat162float(__float2bfloat16_rn(s0)), a1 = __bfloat162float(__float2bfloat16_rn(s1));
         const __nv_bfloat162 o = __floats2bfloat162_rn(__fmul_rn(a0, u0), __fmul_rn(a1, u1));
@@ -103,9 +92,47 @@ __device__ __forceinline__ uint32_t silu_mul_pair(uint32_t g2, uint32_t u2) {
 }
 
 template <bool BF16>
-__device__ __forceinline__ uint4 silu_mul_8(const uint4 g, const uint4 u) {
+__device__ __noinline__ uint4 silu_mul_8_any(uint4 g, uint4 u) {
     return make_uint4(silu_mul_pair<BF16>(g.x, u.x), silu_mul_pair<BF16>(g.y, u.y), silu_mul_pair<BF16>(g.z, u.z),
                       silu_mul_pair<BF16>(g.w, u.w));
+}
+
+// Eight elements: one look at all gates, then the packed form for every pair or (a zero, an infinity, a bfloat16 far below zero
+// among them) the scalar one out of line: a branch and both forms per pair overflowed the instruction cache.
+template <bool BF16>
+__device__ __forceinline__ uint4 silu_mul_8(const uint4 g, const uint4 u) {
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
+    float gf[8];
+    float lo = 3.0e38f, hi = 0.0f, least = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (BF16) {
+            gf[2 * k] = __uint_as_float(gw[k] << 16); gf[2 * k + 1] = __uint_as_float(gw[k] & 0xffff0000u);
+            least = fminf(least, fminf(gf[2 * k], gf[2 * k + 1]));
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&gw[k]));
+            gf[2 * k] = f.x; gf[2 * k + 1] = f.y;
+        }
+        lo = fminf(lo, fminf(fabsf(gf[2 * k]), fabsf(gf[2 * k + 1])));
+        hi = fmaxf(hi, fmaxf(fabsf(gf[2 * k]), fabsf(gf[2 * k + 1])));
+    }
+    if (!(lo > (BF16 ? 8.0e-28f : 0.0f) && hi < 3.0e38f && (!BF16 || least > -80.0f))) return silu_mul_8_any<BF16>(g, u);
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float s0, s1;
+        unpack2(silu2(pack2(gf[2 * k], gf[2 * k + 1])), s0, s1);
+        if (BF16) {
+            const float a0 = __bfloat162float(__float2bfloat16_rn(s0)), a1 = __bfloat162float(__float2bfloat16_rn(s1));
+            const __nv_bfloat162 h = __floats2bfloat162_rn(__fmul_rn(a0, __uint_as_float(uw[k] << 16)), __fmul_rn(a1, __uint_as_float(uw[k] & 0xffff0000u)));
+            o[k] = *reinterpret_cast<const uint32_t *>(&h);
+        } else {
+            // the product of two float16 values is exact in binary32: one rounding, as float16 multiplies
+            const __half2 h = __hmul2(__floats2half2_rn(s0, s1), *reinterpret_cast<const __half2 *>(&uw[k]));
+            o[k] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 }  // namespace flh
