@@ -305,21 +305,6 @@ def rope_kv(qkv, cos, sin, q_out, k_cache, v_cache, B, S, nh, nkv, cur, q_by_tok
     return q_out
 
 
-def rmsnorm(x, weight, eps: float):
-    """RMS-norm over the last dimension of x f16 [.., K] (rows of any stride) with a weight f16 [K]: include/flh_b200.h, flh_b200_rmsnorm_f16."""
-    K = x.shape[-1]
-    _check(x.is_cuda and x.dtype == torch.float16 and weight.dtype == torch.float16 and weight.is_contiguous() and weight.device == x.device,
-           "x and weight must be float16 tensors on one GPU")
-    rows = x.reshape(-1, K)
-    if rows.stride(1) != 1 or rows.stride(0) % 8 or rows.stride(0) < K or rows.data_ptr() % 16:
-        rows = rows.contiguous()
-    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    with _guard(x.device):
-        _lib.check(_lib.load().flh_b200_rmsnorm_f16(_ptr(rows), _ptr(weight), rows.shape[0], K, rows.stride(0) if rows.shape[0] > 1 else K, float(eps),
-                                                    _ptr(out), _stream(x)), "rmsnorm")
-    return out
-
-
 def rmsnorm_quant_token_asym_i4(x, eps: float, hadamard: bool = False, clip: float = 1.0):
     """RMS-norm (weight 1) + per-token asymmetric int4 in one pass, K = 4096 or 8192 (include/flh_b200.h).
     x [M, K] f16/bf16 (row stride allowed) -> (q u8[M,K/2], scale f16[M], zero f16[M])."""

@@ -26,7 +26,6 @@ SIGNATURES = {
     "flh_b200_silu_mul": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_void_p, c_void_p]),
     "flh_b200_silu_mul_quant_token_asym_i4": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_int, c_int, c_void_p, c_float,
                                                       c_void_p, c_void_p, c_void_p, c_void_p]),
-    "flh_b200_rmsnorm_f16": (c_int, [c_void_p, c_void_p, c_long, c_long, c_long, c_float, c_void_p, c_void_p]),
     "flh_b200_rope_kv_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                      c_int, c_int, c_void_p]),
     "flh_b200_rope_kv_by_token_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,

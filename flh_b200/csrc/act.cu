@@ -28,58 +28,6 @@ __global__ void __launch_bounds__(kSiluThreads) silu_mul_kernel(const uint8_t *_
     }
 }
 
-// RMS-norm with a weight: y = half(half(x * 1 / sqrt(mean(x^2) + eps)) * w), the sum of squares in binary32.  One block per row;
-// a row is a few kilobytes, read once and kept in registers (kNormPieces 16-byte pieces a thread).  Stands in for nine tensor
-// operations: 26 us for the 16 rows of a decode step, and four passes over memory for the rows of a prompt.
-constexpr int kNormThreads = 256, kNormPieces = 4;             // rows of up to 8192 values
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const uint4 *__restrict__ x, const uint4 *__restrict__ w, int pieces, long ld16,
-                                                               float eps, float inv_n, uint4 *__restrict__ out) {
-    __shared__ float part[kNormThreads / 32];
-    pdl_wait();
-    pdl_trigger();
-    const uint4 *row = x + blockIdx.x * ld16;
-    uint4 v[kNormPieces];
-    float ssq = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kNormPieces; ++k) {
-        const int i = threadIdx.x + k * kNormThreads;
-        v[k] = i < pieces ? ldg_nc_v4(row + i) : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int k = 0; k < kNormPieces; ++k) {
-        const __half2 *h = reinterpret_cast<const __half2 *>(&v[k]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(h[e]);
-            ssq = __fmaf_rn(f.x, f.x, ssq);
-            ssq = __fmaf_rn(f.y, f.y, ssq);
-        }
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) ssq = __fadd_rn(ssq, __shfl_xor_sync(0xffffffffu, ssq, s));
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ssq;
-    __syncthreads();
-    float total = part[0];
-#pragma unroll
-    for (int k = 1; k < kNormThreads / 32; ++k) total = __fadd_rn(total, part[k]);
-    const float c = __frcp_rn(__fsqrt_rn(__fadd_rn(__fmul_rn(total, inv_n), eps)));
-#pragma unroll
-    for (int k = 0; k < kNormPieces; ++k) {
-        const int i = threadIdx.x + k * kNormThreads;
-        if (i >= pieces) break;
-        const uint4 wv = __ldg(w + i);
-        const __half2 *h = reinterpret_cast<const __half2 *>(&v[k]), *wh = reinterpret_cast<const __half2 *>(&wv);
-        uint4 o;
-        __half2 *oh = reinterpret_cast<__half2 *>(&o);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(h[e]);
-            oh[e] = __hmul2(__floats2half2_rn(__fmul_rn(f.x, c), __fmul_rn(f.y, c)), wh[e]);
-        }
-        out[(long)blockIdx.x * pieces + i] = o;
-    }
-}
-
 struct RopeParams {
     const __half *qkv;         // [B * S, (nh + 2 nkv) * D]
     const float *cos, *sin;    // [S, D / 2] for the S positions of this step
@@ -153,11 +101,6 @@ int launch_silu_mul(const void *gu, int in_dtype, long M, long F, long ld, void 
     if (in_dtype == FLH_B200_BF16)
         return cuda_status(launch_pdl(silu_mul_kernel<true>, grid, kSiluThreads, 0, stream, static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out)), "silu_mul launch");
     return cuda_status(launch_pdl(silu_mul_kernel<false>, grid, kSiluThreads, 0, stream, static_cast<const uint8_t *>(gu), M, F, ld * 2, static_cast<uint8_t *>(out)), "silu_mul launch");
-}
-
-int launch_rmsnorm(const void *x, const void *w, long M, long K, long ld, float eps, void *out, cudaStream_t stream) {
-    return cuda_status(launch_pdl(rmsnorm_kernel, dim3((unsigned)M), kNormThreads, 0, stream, static_cast<const uint4 *>(x), static_cast<const uint4 *>(w),
-                                  (int)(K / 8), ld / 8, eps, 1.0f / (float)K, static_cast<uint4 *>(out)), "rmsnorm launch");
 }
 
 int launch_rope_kv(const void *qkv, const float *cos, const float *sin, void *q_out, void *k_cache, void *v_cache,

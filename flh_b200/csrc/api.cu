@@ -61,7 +61,6 @@ int quant_token_factor_status_clear();
 const char *quant_token_kernel_name(long, long, int, int);
 int launch_silu_mul(const void *, int, long, long, long, void *, cudaStream_t);
 int launch_silu_mul_quant_token_tc(const void *, int, long, long, long, int, const uint32_t *, float, uint8_t *, void *, void *, cudaStream_t);
-int launch_rmsnorm(const void *, const void *, long, long, long, float, void *, cudaStream_t);
 int launch_rope_kv(const void *, const float *, const float *, void *, void *, void *, int, int, int, int, int, int, int, int, cudaStream_t);
 int quant_token_tc_status(int *);
 int launch_gptq_block(const float *, long, const float *, long, const float *, const float *, long, const int *, long, int, int, int,
@@ -204,16 +203,6 @@ int flh_b200_rmsnorm_quant_token_asym_i4(const void *x, int in_dtype, long M, lo
     FLH_REQUIRE(aligned16(x), FLH_B200_EALIGN, "x must be 16-byte aligned");
     FLH_REQUIRE(aligned16(q), FLH_B200_EALIGN, "q must be 16-byte aligned");
     return launch_quant_token_warp(x, in_dtype, M, K, ld, hadamard, eps, clip, q, scale, zero, static_cast<cudaStream_t>(stream));
-}
-
-int flh_b200_rmsnorm_f16(const void *x, const void *weight, long M, long K, long ld, float eps, void *out, void *stream) {
-    FLH_REQUIRE(M >= 0 && M <= 0x7fffffffL && K > 0 && K % 8 == 0 && K <= 8192, FLH_B200_EINVAL, "bad shape M=%ld K=%ld (K must be a multiple of 8, at most 8192)", M, K);
-    FLH_REQUIRE(ld >= K && ld % 8 == 0, FLH_B200_EALIGN, "row stride must be >= K and a multiple of 8 elements (got %ld)", ld);
-    FLH_REQUIRE(eps >= 0.0f, FLH_B200_EINVAL, "eps must be >= 0");
-    if (M == 0) return 0;
-    FLH_REQUIRE(x && weight && out, FLH_B200_EINVAL, "null pointer");
-    FLH_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(out), FLH_B200_EALIGN, "pointers must be 16-byte aligned");
-    return launch_rmsnorm(x, weight, M, K, ld, eps, out, static_cast<cudaStream_t>(stream));
 }
 
 int flh_b200_silu_mul(const void *gu, int in_dtype, long M, long F, long ld, void *out, void *stream) {

@@ -134,10 +134,6 @@ int flh_b200_rmsnorm_quant_group_sym_i4(const void *x, long M, long K, float eps
 
 /* ---- the decoder wiring either side of the quantised linears (flh/quantized_model/modeling_llama.py:389-470, 522-526) ---- */
 
-/* RMS-norm with a weight (flh/nn/normalization.py): out[m, k] = f16(f16(x c) weight[k]), c = 1 / sqrt(mean(x^2) + eps), the sum of
- * squares in binary32.  x f16 [M, K], row stride ld elements (a multiple of 8); out contiguous; K % 8 == 0, K <= 8192. */
-int flh_b200_rmsnorm_f16(const void *x, const void *weight, long M, long K, long ld, float eps, void *out, void *stream);
-
 /* SiLU(gate) * up of the MLP.  gu [M, 2F] f16 or bf16 with row stride ld (elements): gate = columns [0, F), up = columns
  * [F, 2F) — the output of the merged gate/up GEMM; out [M, F] contiguous, same type.  F % 8 == 0, 16-byte aligned pointers.
  * Defined bit for bit (so that the CPU restatement agrees): e = exp32(-g), s = round16(g / (1 + e)), out = round16(s * u),

@@ -141,7 +141,7 @@ def test_rope_by_token_is_the_transposed_form(cuda, D, B, S):
 
 @pytest.mark.parametrize("m,k", [(1, 8), (3, 2056), (16, 4096), (33, 8192)])
 def test_rmsnorm(cuda, m, k):
-    """Binary32 sums in another order and a correctly rounded 1 / sqrt: one ulp of each of the two float16 roundings (2^-10 each)."""
+    """Against 64 bits: one ulp of each of the two float16 roundings (2^-10 each), the binary32 part far below that."""
     from flh_b200.model import RMSNorm
     x = torch.from_numpy(rs(m + k).standard_normal((m, k + 8)).astype(np.float16)).cuda()[:, :k]
     norm = RMSNorm(k, 1e-5).cuda()
@@ -150,6 +150,39 @@ def test_rmsnorm(cuda, m, k):
     want = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5) * norm.weight.double()
     err = (norm(x).double() - want).abs()
     assert bool((err <= 2.0 ** -9 * want.abs() + 2.0 ** -24).all()), err.max().item()
+
+
+def _norm_of(k):
+    from flh_b200.model import RMSNorm
+    norm = RMSNorm(k, 1e-5).cuda()
+    norm.weight.data.copy_(torch.from_numpy(rs(5).uniform(0.5, 2.0, k).astype(np.float16)))
+    return norm, lambda x: (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-5)).to(x.dtype) * norm.weight
+
+
+@pytest.mark.parametrize("m,k", [(1, 8), (1, 4096), (3, 2056), (16, 4096), (700, 4096), (33, 8192)])
+@pytest.mark.parametrize("layout", ["contiguous", "strided", "misaligned"])
+def test_rmsnorm_has_the_bits_of_the_tensor_operations(cuda, m, k, layout):
+    norm, want = _norm_of(k)
+    x = torch.from_numpy(rs(m + k).standard_normal(m * (k + 8) + 1).astype(np.float16)).cuda()
+    x = {"contiguous": x[:m * k].view(m, k), "strided": x[:-1].view(m, k + 8)[:, :k], "misaligned": x[1:1 + m * k].view(m, k)}[layout]
+    assert torch.equal(norm(x).view(torch.int16), want(x).view(torch.int16))
+
+
+def test_rmsnorm_under_tangents_vmap_and_tracing(cuda):
+    norm, want = _norm_of(256)
+    x, t = (torch.from_numpy(rs(s).standard_normal((4, 256)).astype(np.float16)).cuda() for s in (1, 2))
+    y, dy = torch.func.jvp(norm, (x,), (t,))
+    assert torch.equal(y, want(x)) and torch.equal(dy, torch.func.jvp(want, (x,), (t,))[1]) and bool(dy.any())
+    assert torch.equal(torch.vmap(norm)(x), torch.vmap(want)(x))
+    traced = torch.jit.trace(norm, (x,), check_trace=False)
+    assert torch.equal(traced(t), want(t))
+
+
+def test_rmsnorm_refuses_another_width(cuda):
+    norm, _ = _norm_of(256)
+    for k in (128, 512):
+        with pytest.raises(RuntimeError):
+            norm(torch.zeros(2, k, dtype=torch.float16, device="cuda"))
 
 
 @pytest.mark.parametrize("shape", [(128,), (3, 256), (2, 5, 384)])
