@@ -76,9 +76,14 @@ class RMSNorm(torch.nn.Module):
         self.eps = eps
         self.weight = torch.nn.Parameter(torch.ones(dim, dtype=torch.float16), requires_grad=False)
 
-    def forward(self, x):
+    def forward(self, x, last=False):
+        """last: only the last position of x [B, S, K].  The mean is over all positions even then: the order in which a
+        reduction sums a row depends on the number of rows, and the result has the bits of the whole norm's last position."""
         v = x.float()
-        return (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
+        c = torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
+        if last:
+            v, c = v[:, -1:], c[:, -1:]
+        return (v * c).to(x.dtype) * self.weight
 
 
 def rope_tables(pos, d, theta):
@@ -290,5 +295,8 @@ class Decoder(torch.nn.Module):
             x, pre = out if isinstance(out, tuple) else (out, None)
         if sp:
             x = gather_rows(x, None, blocks).view(B, S, -1)
-        # the head reads the last position only: the others need no final norm
-        return self.norm(x) if self.head is None else self.head(self.norm(x[:, -1:]))
+        if self.head is None:
+            return self.norm(x)
+        # the head reads the last position only: the others need no final norm, unless a hook or another module sees it
+        whole = type(self.norm) is not RMSNorm or self.norm._forward_hooks
+        return self.head(self.norm(x)[:, -1:] if whole else self.norm(x, last=True))

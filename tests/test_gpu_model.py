@@ -45,6 +45,23 @@ def test_decode_step_matches_prefill(cuda):
     assert err < 2e-2, err
 
 
+@pytest.mark.parametrize("B,S", [(1, 700), (3, 33), (16, 1)])
+def test_head_input_is_the_last_position_of_the_whole_norm(cuda, B, S):
+    """Bit for bit, and a hook on the norm sees every position."""
+    from flh_b200.model import Decoder, DecoderConfig
+    m = Decoder(DecoderConfig(hidden=4096, n_heads=32, n_kv_heads=32, ffn=512, n_layers=1, vocab=128), torch.device("cuda"), seed=5)
+    seen = {}
+    m.layers[-1].register_forward_hook(lambda mod, args, out: seen.update(x=out))
+    m.head.register_forward_pre_hook(lambda mod, args: seen.update(head=args[0]))
+    ids = torch.randint(0, 128, (B, S), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    m(ids)
+    want = m.norm(seen["x"])
+    assert torch.equal(seen["head"].view(torch.int16), want[:, -1:].view(torch.int16))
+    m.norm.register_forward_hook(lambda mod, args, out: seen.update(norm=out))
+    m(ids)
+    assert torch.equal(seen["norm"].view(torch.int16), want.view(torch.int16)) and torch.equal(seen["head"], want[:, -1:])
+
+
 @pytest.mark.parametrize("mode", ["group_sym", "token_asym"])
 def test_llama7b_shaped_layer_matches_pytorch_twin(cuda, monkeypatch, mode):
     """One decoder layer at the Llama-2-7B shape (hidden 4096, 32 heads, FFN 11008 -> merged QKV at N = 12288, the
