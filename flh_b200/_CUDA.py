@@ -358,21 +358,12 @@ def _workspace(device, stream: int, nbytes: int):
     return ws
 
 
-_SCRATCH: dict = {}
-
-
-def _scratch(device, stream: int, nbytes: int):
-    """Uninitialised scratch for the GEMMs that expand their operands first, one per (device, stream); kept apart from the
-    zeroed split-K workspace, whose counters it would overwrite.  A launch that is being recorded into a graph gets memory
-    of the graph's own instead: the shared buffer is replaced when a larger call comes, the graph would go on using it."""
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    key = (device, stream)
-    ws = _SCRATCH.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _SCRATCH[key] = ws
-    return ws
+def _scratch(device, nbytes: int):
+    """Uninitialised memory for the GEMMs that expand their operands first, of this call alone: the expansion and the GEMM are two
+    launches, and another thread may put its own two on the stream between them.  It comes from what the caching allocator
+    keeps for the current stream (while a graph is recorded, for the graph) and goes back there when the call returns: whoever
+    gets it next runs behind both launches."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def gemm_i4_dequant(A, B, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=None,
@@ -413,7 +404,7 @@ def _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, ag,
         elif zeroed:
             ws = _workspace(A.device, stream, need)        # split-K: zeroed counters, left zeroed
         else:
-            ws = _scratch(A.device, stream, need)          # expanded operands: any contents
+            ws = _scratch(A.device, need)                  # expanded operands: any contents
         _lib.check(lib.flh_b200_gemm_i4_dequant(
             _ptr(A), _ptr(B), _ptr(A_scale), _ptr(A_zero), _ptr(B_scale), _ptr(B_rowsum), _ptr(bias), _ptr(D),
             M, N, K, ag, bg, BF16 if D.dtype == torch.bfloat16 else F16, algo, _ptr(ws), ws.numel() if ws is not None else 0,
@@ -438,7 +429,7 @@ def gemm_i8w_dequant(A, B8, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=N
     D = out if out is not None else torch.empty((M, N), dtype=out_dtype, device=A.device)
     with _guard(A.device):
         stream = _stream(A)
-        ws = _scratch(A.device, stream, M * K)
+        ws = _scratch(A.device, M * K)
         _lib.check(_lib.load().flh_b200_gemm_i8w_dequant(
             _ptr(A), _ptr(B8), _ptr(A_scale), _ptr(A_zero), _ptr(B_scale), _ptr(B_rowsum), _ptr(bias), _ptr(D),
             M, N, K, BF16 if D.dtype == torch.bfloat16 else F16, _ptr(ws), ws.numel(), stream), "gemm_i8w_dequant")

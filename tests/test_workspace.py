@@ -1,0 +1,97 @@
+"""The memory that the GEMM binding hands to the library: who shares it, who keeps it, what happens without it.  The parts that
+need no GPU run on host tensors with a stand-in for the library."""
+import contextlib
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from test_gpu_gemm import _dev, make_case
+
+
+class FakeLibrary:
+    """Takes the GEMM calls, asks for `need` bytes and keeps (algorithm, workspace address, workspace bytes) of each."""
+
+    def __init__(self, need, inside=lambda: None):
+        self.need, self.inside, self.calls = need, inside, []
+
+    def flh_b200_last_error(self):
+        return b""
+
+    def flh_b200_gemm_workspace_bytes(self, *a):
+        return self.need
+
+    def flh_b200_gemm_pick_algo(self, M, *a):
+        return 4 if M <= 64 else 1
+
+    def flh_b200_gemm_i4_dequant(self, *a):
+        self.calls.append((a[14], a[15], a[16]))
+        self.inside()
+        return 0
+
+    def flh_b200_gemm_i8w_dequant(self, *a):
+        self.calls.append((None, a[12], a[13]))
+        self.inside()
+        return 0
+
+
+@pytest.fixture
+def binding(monkeypatch):
+    import flh_b200
+    C = flh_b200._CUDA
+    monkeypatch.setattr(C, "_guard", lambda device: contextlib.nullcontext())
+    monkeypatch.setattr(C, "_stream", lambda t: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+
+    def use(fake):
+        monkeypatch.setattr(flh_b200._lib, "load", lambda: fake)
+        return C
+    return use
+
+
+def _operands(m, n=128, k=256):
+    return (torch.zeros(m, k // 2, dtype=torch.uint8), torch.zeros(n, k // 2, dtype=torch.uint8),
+            torch.zeros(m, k // 128, dtype=torch.float16), torch.zeros(n, k // 128, dtype=torch.float16))
+
+
+@pytest.mark.parametrize("entry", ["gemm_i4_dequant", "gemm_i8w_dequant"])
+def test_calls_in_flight_have_scratch_of_their_own(binding, entry):
+    """A prefill GEMM is two launches that meet in its scratch; two threads inside the library at once must not share it."""
+    both = threading.Barrier(2, timeout=60)
+    fake = FakeLibrary(4096, both.wait)
+    C = binding(fake)
+    A, B, SA, SB = _operands(100)
+    if entry == "gemm_i8w_dequant":
+        B = torch.zeros(128, 256, dtype=torch.uint8)
+    threads = [threading.Thread(target=lambda: getattr(C, entry)(A, B, SA, SB)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    (_, p0, n0), (_, p1, n1) = fake.calls
+    assert p0 and p1 and (p0 + n0 <= p1 or p1 + n1 <= p0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("groups,m,n", [((128, 128, False), 300, 512), ((0, 0, True), 1536, 256)])
+def test_two_threads_on_one_stream(cuda, groups, m, n):
+    """Different operands from two threads on the default stream: every result is that of its own operands."""
+    k, wrong = 2048, []
+    work = []
+    for seed in (1, 2):
+        ap, bp, sa, sb, za, _ = make_case(seed, m, n, k, *groups)
+        A, B, SA, SB = (_dev(t) for t in (ap, bp, sa, sb))
+        kw = {} if za is None else {"A_zero": _dev(za), "B_rowsum": cuda.weight_rowsum(B, k)}
+        work.append(((A, B, SA, SB), kw, _dev(O.gemm_i4_dequant(ap, bp, sa, sb, a_zero=za).view(np.int16))))
+
+    def loop(args, kw, want):
+        got = [cuda.gemm_i4_dequant(*args, **kw) for _ in range(200)]
+        wrong.append(sum(not torch.equal(d.view(torch.int16), want) for d in got))
+    threads = [threading.Thread(target=loop, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert wrong == [0, 0]
