@@ -404,7 +404,12 @@ def _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, ag,
         elif zeroed:
             ws = _workspace(A.device, stream, need)        # split-K: zeroed counters, left zeroed
         else:
-            ws = _scratch(A.device, need)                  # expanded operands: any contents
+            try:
+                ws = _scratch(A.device, need)              # expanded operands: any contents
+            except torch.OutOfMemoryError:
+                if algo != GEMM_AUTO:
+                    raise
+                ws = None                                  # AUTO has a kernel that converts inside, with the same results
         _lib.check(lib.flh_b200_gemm_i4_dequant(
             _ptr(A), _ptr(B), _ptr(A_scale), _ptr(A_zero), _ptr(B_scale), _ptr(B_rowsum), _ptr(bias), _ptr(D),
             M, N, K, ag, bg, BF16 if D.dtype == torch.bfloat16 else F16, algo, _ptr(ws), ws.numel() if ws is not None else 0,

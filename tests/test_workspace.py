@@ -74,6 +74,22 @@ def test_calls_in_flight_have_scratch_of_their_own(binding, entry):
     assert p0 and p1 and (p0 + n0 <= p1 or p1 + n1 <= p0)
 
 
+def test_auto_does_without_scratch_that_cannot_be_had(binding, monkeypatch):
+    fake = FakeLibrary(4096)
+    C = binding(fake)
+    args, real = _operands(100), torch.empty
+
+    def empty(*a, dtype=None, **kw):
+        if dtype is torch.uint8:
+            raise torch.OutOfMemoryError("no memory")
+        return real(*a, dtype=dtype, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+    C.gemm_i4_dequant(*args)
+    assert fake.calls == [(0, None, 0)]
+    with pytest.raises(torch.OutOfMemoryError):
+        C.gemm_i4_dequant(*args, algo=C.GEMM_GROUP_F8)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("groups,m,n", [((128, 128, False), 300, 512), ((0, 0, True), 1536, 256)])
 def test_two_threads_on_one_stream(cuda, groups, m, n):
