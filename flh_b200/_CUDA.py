@@ -348,8 +348,14 @@ _WORKSPACES: dict = {}
 
 
 def _workspace(device, stream: int, nbytes: int):
-    """Zero-initialised scratch for the split-K decode kernel, one per (device, stream): launches on one
-    stream run in order, so they may share it; the kernel leaves its counters zeroed."""
+    """Scratch for the decode kernels that share tiles, arrival counters (the first 4 KB) zero, one per (device, stream): launches
+    on one stream run in order, so they may share it; a launch leaves its counters zeroed.  A launch that is being recorded
+    gets memory of the graph's own, zeroed on every replay: the shared buffer is replaced when a larger call comes, and the
+    graph may be replayed beside calls that use it."""
+    if torch.cuda.is_current_stream_capturing():
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        ws[:4096].zero_()
+        return ws
     key = (device, stream)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:

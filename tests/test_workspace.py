@@ -1,6 +1,7 @@
 """The memory that the GEMM binding hands to the library: who shares it, who keeps it, what happens without it.  The parts that
 need no GPU run on host tensors with a stand-in for the library."""
 import contextlib
+import ctypes
 import threading
 
 import numpy as np
@@ -88,6 +89,47 @@ def test_auto_does_without_scratch_that_cannot_be_had(binding, monkeypatch):
     assert fake.calls == [(0, None, 0)]
     with pytest.raises(torch.OutOfMemoryError):
         C.gemm_i4_dequant(*args, algo=C.GEMM_GROUP_F8)
+
+
+def test_recorded_decode_call_keeps_off_the_shared_workspace(binding, monkeypatch):
+    counters = []
+    fake = FakeLibrary(16384, lambda: counters.append(bytes((ctypes.c_uint8 * 4096).from_address(fake.calls[-1][1]))))
+    C = binding(fake)
+    monkeypatch.setattr(C, "_WORKSPACES", {})
+    args = _operands(16)
+    for capturing in (True, False, True):
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+        C.gemm_i4_dequant(*args)
+        assert len(C._WORKSPACES) == (len(counters) > 1)            # a recorded call leaves nothing for the others
+    (shared,) = C._WORKSPACES.values()
+    assert fake.calls[1][1] == shared.data_ptr() != fake.calls[2][1] and not any(map(any, counters))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("warm", [True, False])
+def test_recorded_decode_call_outlives_a_larger_call(cuda, warm):
+    """The larger call replaces the stream's workspace; other tensors get its memory; the recorded call must not care."""
+    m = 64
+    t = [_dev(x) for x in make_case(31, m, 12288, 4096, 128, 128, False)[:4]]
+    large = [_dev(x) for x in make_case(32, m, 57344, 8192, 128, 128, False)[:4]]
+    want, want_large = cuda.gemm_i4_dequant(*t), cuda.gemm_i4_dequant(*large)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        if warm:
+            cuda.gemm_i4_dequant(*t)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            d = cuda.gemm_i4_dequant(*t)
+        assert torch.equal(cuda.gemm_i4_dequant(*large), want_large)
+        junk = [torch.full((10 << 20,), 255, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        for _ in range(2):
+            d.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(d, want)
+    assert all(bool((j == 255).all()) for j in junk)
 
 
 @pytest.mark.gpu
