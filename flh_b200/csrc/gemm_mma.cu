@@ -402,8 +402,9 @@ gemm_stream_kernel(const GemmParams p) {
         st_begin = blockIdx.y * per;
         st_end = min(KB2, st_begin + per);
     }
-    // 4-byte copies of two adjacent f16 scales need an even number of groups per row
-    const bool pair_ok = (KB & 1) == 0;
+    // copies of two adjacent scales (4 bytes) or row sums (8) need an even number of groups per row and arrays that start on such a boundary
+    const bool pair_ok = (KB & 1) == 0 && ((reinterpret_cast<uintptr_t>(p.a_scale) | reinterpret_cast<uintptr_t>(p.a_zero) | reinterpret_cast<uintptr_t>(p.b_scale)) & 3) == 0 &&
+                         (reinterpret_cast<uintptr_t>(p.b_rowsum) & 7) == 0;
 
     auto load_stage = [&](int stage, int kb2) {
         uint8_t *st = smem + stage * Plan::kStage;

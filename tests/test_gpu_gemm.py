@@ -164,6 +164,24 @@ def test_auto_picks_decode_tc_for_large_decode_shapes(cuda):
     assert pick(128, 8192, 8192, 128, 128) == TC
 
 
+def _off(t, front):
+    """The same values in an array that starts `front` elements behind an allocation's boundary."""
+    return torch.cat((t.flatten()[:front], t.flatten()))[front:].view(t.shape)
+
+
+@pytest.mark.parametrize("algo", [STREAM, SPLITK])
+@pytest.mark.parametrize("mode", [(128, 128, False), (128, 128, True), (0, 128, True), (128, 0, False)])
+@pytest.mark.parametrize("m", [3, 16, 40])
+def test_streaming_kernel_takes_scales_at_any_element(cuda, algo, mode, m):
+    """float16 scales and zero-points two bytes off a word, int32 row sums four bytes off a pair: the same bits as aligned ones."""
+    ap, bp, sa, sb, za, _ = make_case(41 * m, m, 512, 2048, *mode)
+    A, B, SA, SB = _dev(ap), _dev(bp), _dev(sa), _dev(sb)
+    kw = {} if za is None else {"A_zero": _dev(za), "B_rowsum": cuda.weight_rowsum(B, 128)}
+    want = cuda.gemm_i4_dequant(A, B, SA, SB, algo=algo, **kw)
+    got = cuda.gemm_i4_dequant(A, B, _off(SA, 1), _off(SB, 1), algo=algo, **{k: _off(t, 1) for k, t in kw.items()})
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 def test_reference_script_case(cuda):
     # test/test_gemm_dequant.py: M=1, N=1024, K=2048, signed codes, N(0,1)-like scales of both signs
     run_case(cuda, STREAM, make_case(0, 1, 1024, 2048, 128, 128, False, neg_scales=True))
