@@ -391,20 +391,27 @@ def gemm_i4_dequant(A, B, A_scale, B_scale, A_zero=None, B_rowsum=None, bias=Non
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_plan(lib, M, N, K, ag, bg, algo, has_zero):
-    """(workspace bytes, whether it must be zeroed) of a GEMM: a function of the sizes alone."""
+def _gemm_plan(lib, M, N, K, ag, bg, algo, has_zero, words):
+    """(algorithm, workspace bytes, whether they must be zeroed) of a GEMM: a function of the sizes and of whether the scales are
+    aligned to 4 bytes."""
+    picked = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
+    zeroed = M <= 64 and picked not in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_GROUP_F8)
     # what AUTO can use depends on the zero-points only where there are group scales: those keep the kernels without workspace of that kind
-    auto = algo == GEMM_AUTO and not (has_zero and min(ag, bg) < K)
-    need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE if auto else algo)
-    resolved = algo if algo != GEMM_AUTO else lib.flh_b200_gemm_pick_algo(M, N, K, ag, bg)
-    return need, M <= 64 and resolved not in (GEMM_TCGEN05_I8, GEMM_TCGEN05_I8_PAIR, GEMM_GROUP_F8)
+    if algo == GEMM_AUTO and not (has_zero and min(ag, bg) < K):
+        need = lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, GEMM_AUTO_WORKSPACE)
+        if need or picked not in (GEMM_STREAM_SPLITK, GEMM_DECODE_TC):
+            return algo, need, zeroed
+        if words or min(ag, bg) == K:
+            return GEMM_DECODE_RING, 0, False
+    return algo, lib.flh_b200_gemm_workspace_bytes(M, N, K, ag, bg, algo), zeroed
 
 
 def _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, ag, bg, algo):
     lib = _lib.load()
     with _guard(A.device):
         stream = _stream(A)
-        need, zeroed = _gemm_plan(lib, M, N, K, ag, bg, algo, A_zero is not None)
+        words = (A_scale.data_ptr() | B_scale.data_ptr()) % 4 == 0
+        algo, need, zeroed = _gemm_plan(lib, M, N, K, ag, bg, algo, A_zero is not None, words)
         if not need:
             ws = None
         elif zeroed:

@@ -316,8 +316,9 @@ int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) 
 //   35.0 -> 26.6; 64 tokens: 4096 -> 4096 18.1 -> 10.2, but 11008 -> 4096 19.9 -> 20.7 and 8192 -> 28672 48.5 -> 57.5 (its
 //   mma.sync rate is the limit there): above 32 tokens for weights below 20 MiB;
 //   group scales, 16 tokens: 4096 -> 4096 9.0 -> 5.5, 11008 -> 4096 15.3 -> 11.0, 8192 -> 28672 43.1 -> 39.0; 32 tokens: 12.0 -> 7.5,
-//   21.0 -> 14.9, but 55.3 -> 57.8: above 16 tokens for weights below 64 MiB; 64 tokens: never.  Where the plain streaming
-//   kernel is what AUTO ran, AUTO's results are a single binary32 chain bit for bit and stay so.
+//   21.0 -> 14.9, but 55.3 -> 57.8: above 16 tokens for weights below 64 MiB; 64 tokens: never.  With group scales it adds the
+//   binary32 chains of its warps, so it stands in only for kernels that split the chain too, and in AUTO only where the caller
+//   handed over the workspace that they need: without one AUTO's results are a single chain bit for bit.
 static bool decode_ring_pays(long M, long N, long K, long a_group, long b_group, bool zero) {
     const bool grouped = (a_group < b_group ? a_group : b_group) < K;
     if (!gemm_decode_ring_supported(M, N, K, grouped, zero)) return false;
@@ -364,8 +365,11 @@ int flh_b200_gemm_i4_dequant(const uint8_t *A, const uint8_t *B, const void *a_s
     }
     const bool grouped = gmin < K;
     // (it reads the scales of two groups as one word)
-    const bool words = ((reinterpret_cast<uintptr_t>(a_scale) | reinterpret_cast<uintptr_t>(b_scale)) & 3) == 0;
-    if (algo == FLH_B200_GEMM_AUTO && words && decode_ring_pays(M, N, K, a_group, b_group, a_zero != nullptr)) algo = FLH_B200_GEMM_DECODE_RING;
+    const bool words = !grouped || ((reinterpret_cast<uintptr_t>(a_scale) | reinterpret_cast<uintptr_t>(b_scale)) & 3) == 0;
+    if (algo == FLH_B200_GEMM_AUTO && words && decode_ring_pays(M, N, K, a_group, b_group, a_zero != nullptr) &&
+        (!grouped || (workspace && workspace_bytes >= flh_b200_gemm_workspace_bytes(M, N, K, a_group, b_group, FLH_B200_GEMM_AUTO) &&
+                      (reinterpret_cast<uintptr_t>(workspace) & 255) == 0)))
+        algo = FLH_B200_GEMM_DECODE_RING;
     if (algo == FLH_B200_GEMM_AUTO) {
         algo = flh_b200_gemm_pick_algo(M, N, K, a_group, b_group);
         // without (enough) scratch the tensor-core decode kernel gives way to the streaming kernels

@@ -57,8 +57,10 @@ extern "C" {
                                     workspace, two-CTA tcgen05 kernel with exact binary32 group sums; N % 256 == 0 */
 #define FLH_B200_GEMM_DECODE_RING 11 /* M <= 64: weights through a TMA ring, mma.sync, K split over the warps of a CTA; no workspace.
                                      AUTO runs it before what flh_b200_gemm_pick_algo names: without group scales up to 32
-                                     tokens (64 for small weights), with them in place of SPLITK and DECODE_TC up to 16 (32) */
-#define FLH_B200_GEMM_AUTO_WORKSPACE 10 /* only for flh_b200_gemm_workspace_bytes: the most workspace AUTO can make use of */
+                                     tokens (64 for small weights); with them up to 16 (32), in place of SPLITK and DECODE_TC
+                                     and only when handed the workspace of those */
+#define FLH_B200_GEMM_AUTO_WORKSPACE 10 /* only for flh_b200_gemm_workspace_bytes: what the fastest kernel for the shape needs.  0 for
+                                     decode shapes for which GEMM_AUTO is not 0 too: that kernel is DECODE_RING, to be named */
 
 int flh_b200_version(void);
 const char *flh_b200_last_error(void);
@@ -207,10 +209,13 @@ int flh_b200_weight_rowsum(const uint8_t *B, long N, long K, long group, int32_t
  *   the packed weights reach 64 MiB, 32 MiB above 16 tokens, 12 MiB above 32).  Its first 4 KB are arrival
  *   counters that must be ZERO before the first launch and are left zero by every launch; launches that
  *   share a workspace must not overlap on the GPU.  With AUTO and no (or too small a) workspace the plain
- *   streaming kernel (or, for large batches, the converting tcgen05 kernel) runs instead.  Both kernels add
+ *   streaming kernel (or, for large batches, the converting tcgen05 kernel) runs instead, with group scales (without
+ *   them the ring kernel may, with the same results).  Both kernels add
  *   the binary32 chains of the CTAs that share a tile in K order, so with group scales their outputs can
  *   differ from the single chain in the last bit (<= 1e-3 relative, the same bits on every run); without
- *   group scales the partial sums are int32 and the result is identical.  STREAM and TCGEN05 never split a chain.
+ *   group scales the partial sums are int32 and the result is identical.  DECODE_RING adds the chains of its warps in
+ *   the same way; it needs no workspace and, with group scales, scales aligned to 4 bytes.  STREAM and TCGEN05 never
+ *   split a chain.
  *   The int8-operand kernels (TCGEN05_I8, TCGEN05_I8_PAIR; a_group = b_group = K only) write the expanded
  *   operands, (M + N) * K bytes, into the workspace; it needs no initial contents, results are bit-identical
  *   to the other kernels, and launches that share a workspace must not overlap on the GPU.

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from test_gpu_gemm import _dev, make_case
+from test_gpu_gemm import _dev, _off, make_case
 
 
 class FakeLibrary:
@@ -153,3 +153,42 @@ def test_two_threads_on_one_stream(cuda, groups, m, n):
     for t in threads:
         t.join()
     assert wrong == [0, 0]
+
+
+def _auto(cuda, t, workspace, nbytes):
+    m, n, k = t[0].shape[0], t[1].shape[0], 2 * t[0].shape[1]
+    d = torch.empty(m, n, dtype=torch.float16, device="cuda")
+    rc = cuda._lib.load().flh_b200_gemm_i4_dequant(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), None, t[3].data_ptr(), None, None, d.data_ptr(), m, n, k,
+                                                   k // t[2].shape[1], k // t[3].shape[1], 0, 0, workspace, nbytes, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return d
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (16, 4096, 11008), (31, 4096, 4096)])
+def test_auto_without_workspace_is_the_single_chain(cuda, m, n, k):
+    """Whoever passes no workspace, the reference's own symbol among them, gets the chain of the oracle bit for bit; with the
+    workspace of the kernels that split the chain AUTO may take the ring kernel."""
+    case = make_case(m + n, m, n, k, 128, 128, False)
+    t, want = [_dev(x) for x in case[:4]], _dev(O.gemm_i4_dequant(*case[:4]).view(np.int16))
+    lib, ring = cuda._lib.load(), cuda.gemm_i4_dequant(*t, algo=cuda.GEMM_DECODE_RING)
+    need = lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, 0)
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    assert torch.equal(_auto(cuda, t, None, 0).view(torch.int16), want)
+    assert torch.equal(_auto(cuda, t, ws.data_ptr(), need), ring) and torch.equal(cuda.gemm_i4_dequant(*t), ring)
+    d = torch.empty(m, n, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    lib.flhDenseLayerGEMM_i4_o16(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(), d.data_ptr(), m, n, k)
+    torch.cuda.synchronize()
+    assert torch.equal(d.view(torch.int16), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [16, 64])
+def test_scales_off_a_word_boundary_keep_the_workspace(cuda, m):
+    """The ring kernel reads group scales as words; others go to the kernel that pick_algo names, with its workspace."""
+    t = [_dev(x) for x in make_case(9, m, 4096, 4096, 128, 128, False)[:4]]
+    named = cuda._lib.load().flh_b200_gemm_pick_algo(m, 4096, 4096, 128, 128)
+    assert torch.equal(cuda.gemm_i4_dequant(*t[:2], _off(t[2], 1), _off(t[3], 1)), cuda.gemm_i4_dequant(*t, algo=named))
+    u = [_dev(x) for x in make_case(9, m, 4096, 4096, 0, 0, False)[:4]]
+    assert torch.equal(cuda.gemm_i4_dequant(*u[:2], _off(u[2], 1), _off(u[3], 1)), cuda.gemm_i4_dequant(*u, algo=named))
