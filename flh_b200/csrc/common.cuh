@@ -32,8 +32,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may start while the one before it on the stream still runs
 // (once every CTA of that one has called pdl_trigger or left).  The rules that keep it safe:
-//   * nothing that an earlier kernel wrote is read, and nothing is written, before pdl_wait — which returns when the kernel
-//     before has completed, and with it, because it waited too, everything before that;
+//   * nothing that an earlier kernel wrote is relied on, and nothing is written, before pdl_wait — which returns when the kernel
+//     before has completed, and with it, because it waited too, everything before that.  (The tensor-core quantiser reads its
+//     factor table before, and compares it after; the ring GEMM prefetches weights into the L2 cache before.)
 //   * pdl_trigger comes after pdl_wait (or in a kernel launched normally), and in a kernel that uses tensor memory after its
 //     allocation: a dependent that allocates must never stand in front of the kernel it waits for.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -103,6 +103,7 @@ quant_token_asym_kernel(const TokenParams p) {
     const int lane = t & 31, warp = t >> 5;
     const bool active = t < p.T;
 
+    pdl_wait();                              // before anything is read, the sign matrix included
     // Tensor-core factor stage: the sign matrix lives in shared memory for the whole (persistent) CTA,
     // rows padded by 16 bytes so that ldmatrix reads are conflict-free.
     const int smat_ld = p.kp + 8;                                              // bf16 elements per row
@@ -117,7 +118,6 @@ quant_token_asym_kernel(const TokenParams p) {
         __syncthreads();
     }
 
-    pdl_wait();
     pdl_trigger();
     for (long row = blockIdx.x; row < p.M; row += gridDim.x) {
     float x[64];

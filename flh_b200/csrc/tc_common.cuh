@@ -93,6 +93,13 @@ __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// the same barrier; true for all when v is for any
+__device__ __forceinline__ bool bar_or_named(int id, int nthreads, bool v) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"(id), "r"(nthreads), "r"((int)v) : "memory");
+    return r != 0;
+}
 
 // K-major, 128-byte swizzle: 8-row groups 1024 B apart (SBO), LBO unused (1), descriptor version 1.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {

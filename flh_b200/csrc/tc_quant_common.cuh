@@ -25,16 +25,19 @@ __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
     asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
     return r;
 }
+
 // A = G (or diag(G, G) when two token rows share an MMA: R == 2) as a K-major tcgen05 operand with the 128-byte swizzle:
 // element (m, k) lies in K atom kb = k / 64 at (kb * Mtot / 8 + m / 8) * 1024, row m % 8 of 128 bytes, 16-byte chunk
 // ((k % 64) / 8) ^ (m % 8).  G[p'][p] = S[a'][a] * (-1)^popc(b' & b) with p = a * B + b (B a power of two, S the kfac x kfac
 // factor given as bit rows, 1 = negative): per row the signs of the factor come as one bit row of the table (staged in
-// shared memory at `sgn` first), the Sylvester part is a parity.  Contains a __syncthreads(): called by the whole CTA.
+// shared memory at `sgn` first, past the L1 cache: it may be read a second time), the Sylvester part is a parity.  `sync` is a
+// barrier of the `nthreads` threads that share the work.
+template <typename Sync>
 __device__ __forceinline__ void build_sign_operand(uint8_t *sm, uint32_t *sgn, const uint32_t *sign_bits, int kfac, int words, int P, int B,
-                                                   int R, int Kdim, int Mtot, bool bf16, int tid, int nthreads) {
+                                                   int R, int Kdim, int Mtot, bool bf16, int tid, int nthreads, Sync sync) {
     if (sign_bits)
-        for (int i = tid; i < kfac * words; i += nthreads) sgn[i] = sign_bits[i];
-    __syncthreads();
+        for (int i = tid; i < kfac * words; i += nthreads) sgn[i] = __ldcg(sign_bits + i);
+    sync();
     const int katoms = (Kdim + 63) >> 6;
     const int cpr = katoms * 8;                                         // 16-byte chunks per row of A
     const int chunks = Mtot * cpr;

@@ -295,6 +295,35 @@ def test_token_asym_full_size_property(cuda):
     assert np.all(np.abs(deq - y) <= 0.51 * s[idx].astype(np.float32)[:, None])
 
 
+@pytest.mark.parametrize("m,k,hadamard,off", [(1, 11008, 1, 0), (300, 11008, 1, 0), (40, 14336, 1, 0), (8, 28672, 1, 0), (5, 11008, 2, 0), (5, 11008, 1, 8)])
+@pytest.mark.parametrize("rows", [16, 4096])
+def test_sign_table_written_by_the_kernel_before(cuda, m, k, hadamard, off, rows):
+    """A factor table in stream order: the expansion kernel, which lets its dependents start early, writes it (any bits will do for
+    a table of signs) over zeros, directly in front of the quantiser."""
+    from flh_b200.hadamard import get_hadK
+    lib, kfac = cuda._lib.load(), get_hadK(k)[1]
+    width = 8192
+    packed = torch.randint(0, 256, (rows, width // 2), dtype=torch.uint8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(k + rows))
+    if off:                                          # codes off a 16-byte boundary: the kernel that reads the bfloat16 matrix behind the bit rows
+        packed.fill_(0xC4)                           # bytes 0x40 and 0xC0 in runs of 16: entries of 3 and -6
+    table = torch.zeros(rows, width, dtype=torch.uint8, device="cuda")
+    sign_bits = table.data_ptr() + table.numel() - (lib.flh_b200_sign_table_bytes(kfac) + 255) // 256 * 256       # the last bytes written
+    x = _dev(activations(k, m, k))
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(wait):
+        q, s, z = (torch.empty(n, dtype=t, device="cuda") for n, t in ((m * k // 2 + off, torch.uint8), (m, torch.float16), (m, torch.float16)))
+        table.zero_()
+        assert lib.flh_b200_expand_i4(packed.data_ptr(), rows, width, table.data_ptr(), stream) == 0
+        if wait:
+            torch.cuda.synchronize()
+        assert lib.flh_b200_quant_token_asym_i4(x.data_ptr(), 0, m, k, k, hadamard, kfac, sign_bits, 1.0, q.data_ptr() + off, s.data_ptr(), z.data_ptr(), stream) == 0
+        return q[off:], s.view(torch.int16), z.view(torch.int16)
+    want = call(True)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(call(False), want))
+
+
 def test_argument_errors(cuda):
     x = torch.zeros((4, 128), dtype=torch.float16, device="cuda")
     with pytest.raises(RuntimeError):
