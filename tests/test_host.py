@@ -49,6 +49,16 @@ def test_argument_validation_without_a_device():
     assert lib.flh_b200_gemm_pick_algo(2048, 4096, 4096, 128, 128) == 1
 
 
+@pytest.mark.parametrize("m,n,k,expands", [(16384, 256, 8192, False), (16384, 256, 4096, False), (16384, 512, 512, False), (384, 12288, 4096, False),
+                                           (8192, 256, 8192, True), (16384, 512, 8192, True), (512, 12288, 4096, True), (65, 4096, 11008, True)])
+def test_auto_expands_group_scale_operands_where_that_was_measured_faster(m, n, k, expands):
+    """The expansion is paid for by the rows of both operands: many rows on a narrow output are as dear as many weights."""
+    from flh_b200 import _lib
+    lib = _lib.load()
+    need = lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, 10)
+    assert need == (lib.flh_b200_gemm_workspace_bytes(m, n, k, 128, 128, 9) if expands else 0)
+
+
 def test_pack_signs_host_helper():
     from flh_b200 import _lib
     from flh_b200.hadamard import get_hadK
