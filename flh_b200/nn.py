@@ -267,7 +267,7 @@ class LinearFLH(torch.nn.Module):
         ga, gb = self.in_features // a_scale.shape[1], self.in_features // w_scale.shape[1]
         rs = None
         if a_zero is not None:
-            if not a_zero.is_contiguous():
+            if a_zero.dim() != 2 or a_zero.shape[0] != M or not a_zero.is_contiguous():
                 a_zero = a_zero.reshape(M, -1)
             rs = self.w_rowsum(min(ga, gb))
         if x.dim() != 2 or M == 0:

@@ -75,6 +75,22 @@ def test_calls_in_flight_have_scratch_of_their_own(binding, entry):
     assert p0 and p1 and (p0 + n0 <= p1 or p1 + n1 <= p0)
 
 
+def test_linear_refuses_zero_points_that_are_not_a_row_each(binding, monkeypatch):
+    """Three tokens with one zero-point: an error, not a read past the end of the array."""
+    from flh_b200.nn import LinearFLH
+    fake = FakeLibrary(0)
+    binding(fake)
+    monkeypatch.setattr(LinearFLH, "w_rowsum", lambda self, group: torch.zeros(128, 256 // group, dtype=torch.int32))
+    lin = LinearFLH(256, 128, dtype=torch.float16, group_size=-1)
+    codes, scale = torch.zeros(3, 128, dtype=torch.uint8), torch.zeros(3, 1, dtype=torch.float16)
+    with pytest.raises(RuntimeError):
+        lin(codes, scale, torch.zeros(1, 1, dtype=torch.float16))
+    assert not fake.calls
+    for zero in (torch.zeros(3, 1), torch.zeros(1, 3, 1), torch.zeros(3, 2)[:, :1]):
+        assert lin(codes, scale, zero.half()).shape == (3, 128)
+    assert len(fake.calls) == 3
+
+
 def test_auto_does_without_scratch_that_cannot_be_had(binding, monkeypatch):
     fake = FakeLibrary(4096)
     C = binding(fake)
