@@ -119,7 +119,7 @@ def act_quant_group(x, gs: int, hadamard: bool):
     normalised transform (the kernel's is un-normalised)."""
     lead, K = x.shape[:-1], x.shape[-1]
     _check(gs in (32, 64, 128), "group_size must be 32, 64, or 128")
-    _check(K % gs == 0, "the last dimension must be a multiple of group_size")
+    _check(K % gs == 0 or x.numel() == 0, "the last dimension must be a multiple of group_size")
     if not x.is_contiguous():
         x = x.reshape(-1, gs)
     _check(x.is_cuda, "Input tensor must be on CUDA")

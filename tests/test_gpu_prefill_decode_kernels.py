@@ -207,3 +207,13 @@ def test_quantiser_module_shapes_and_strides(cuda, shape, kind):
         assert q.shape == shape[:-1] + (K // 2,) and torch.equal(q.reshape(-1), q0.reshape(-1)) and torch.equal(s.reshape(-1), s0.reshape(-1))
     with pytest.raises(RuntimeError):
         ActQuantizer(bits=4, group_size=128, sym=True, use_hadamard=False, packed_output=True)(torch.zeros(2, 192, device="cuda").half())
+
+
+@pytest.mark.parametrize("kind", ["group", "group_had", "token"])
+@pytest.mark.parametrize("shape", [(0, 64), (2, 0, 256)])
+def test_quantiser_module_on_no_rows(cuda, kind, shape):
+    from flh_b200.nn import ActQuantizer
+    sym = kind != "token"
+    quant = ActQuantizer(bits=4, group_size=128 if sym else -1, sym=sym, use_hadamard=kind == "group_had", packed_output=True)
+    s, z, q = quant(torch.empty(shape, dtype=torch.float16, device="cuda"))
+    assert q.shape == shape[:-1] + (shape[-1] // 2,) and s.shape == shape[:-1] + (shape[-1] // 128 if sym else 1,) and (z is None) == sym
