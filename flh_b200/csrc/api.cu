@@ -23,6 +23,7 @@ int fail(int code, const char *fmt, ...) {
 int cuda_status(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return 0;
     set_error("%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
+    cudaGetLastError();                  // reported here: the next launch asks for the last error and must not find this one
     return -(int)e;
 }
 

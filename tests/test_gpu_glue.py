@@ -87,3 +87,23 @@ def test_rope_kv_equals_the_tensor_operations(cuda, B, S, nh, nkv, cur, T):
     keep = torch.ones(T, dtype=torch.bool, device="cuda")
     keep[cur:cur + S] = False
     assert torch.equal(kc[:, :, keep], kc0[:, :, keep]) and torch.equal(vc[:, :, keep], vc0[:, :, keep])
+
+
+def test_a_failed_launch_is_reported_once(cuda):
+    """A launch into a capture that was invalidated fails on the host; the next call, on another stream, must not report it again."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    lib = cuda._lib.load()
+    gu, packed = torch.zeros(4, 512, dtype=torch.float16, device="cuda"), torch.zeros(4, 128, dtype=torch.uint8, device="cuda")
+    out, wide = torch.empty(4, 256, dtype=torch.float16, device="cuda"), torch.empty(4, 256, dtype=torch.uint8, device="cuda")
+    err, stream = rt.cudaStreamCreate()
+    assert err == rt.cudaError_t.cudaSuccess
+    torch.cuda.synchronize()
+    try:
+        rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)
+        assert rt.cudaStreamSynchronize(stream)[0] != rt.cudaError_t.cudaSuccess            # not allowed while capturing: the capture is void
+        assert lib.flh_b200_silu_mul(gu.data_ptr(), 0, 4, 256, 512, out.data_ptr(), int(stream)) < 0
+        rt.cudaStreamEndCapture(stream)
+        assert lib.flh_b200_expand_i4(packed.data_ptr(), 4, 256, wide.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0, lib.flh_b200_last_error()
+        torch.cuda.synchronize()
+    finally:
+        rt.cudaStreamDestroy(stream)
