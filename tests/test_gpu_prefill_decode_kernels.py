@@ -119,6 +119,31 @@ def test_silu_of_every_gate(cuda, bf16):
     assert np.array_equal(got, want.view(np.uint16))
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+def test_silu_of_every_gate_among_ordinary_ones(cuda, bf16):
+    """A group of eight takes the packed form unless one of its gates is out of that form's range: every 16-bit gate, NaN
+    included, in a group whose other seven are ordinary, so that each value meets the form that data sends it to; up runs
+    over ordinary, tiny, huge, zero, infinite and NaN values.  All results bit for bit (any NaN for a NaN)."""
+    f32 = (lambda b: O.bf16_bits_to_f32(b)) if bf16 else (lambda b: b.view(np.float16).astype(np.float32))
+    n = 65536
+    gate = rs(8).standard_normal((n, 8)).astype(np.float32) * 3.0
+    gate = O.f32_to_bf16_bits(gate) if bf16 else gate.astype(np.float16).view(np.uint16)
+    gate[np.arange(n), rs(9).randint(0, 8, n)] = rs(10).permutation(n).astype(np.uint16)
+    gate = gate.reshape(64, -1)
+    with np.errstate(over="ignore", invalid="ignore"):
+        special = np.array([1.0, -2.75, 1e-7, -1e-30, 6e4, 3e38, 0.0, -0.0, np.inf, np.nan], np.float32)
+        special = O.f32_to_bf16_bits(special) if bf16 else special.astype(np.float16).view(np.uint16)
+        up = special[rs(11).randint(0, 10, gate.shape)]
+        gu = np.concatenate([gate, up], axis=1)
+        want = O.silu_mul16(gu if bf16 else gu.view(np.float16), bf16=bf16).view(np.uint16)
+    x = torch.from_numpy(gu.view(np.int16)).cuda().view(torch.bfloat16 if bf16 else torch.float16)
+    got = cuda.silu_mul(x).view(torch.int16).cpu().numpy().view(np.uint16)
+    nan = np.isnan(f32(want))
+    assert np.array_equal(np.isnan(f32(got)), nan)
+    bad = (got != want) & ~nan
+    assert not bad.any(), [(hex(g), hex(u), hex(a), hex(b)) for g, u, a, b in zip(gate[bad][:8], up[bad][:8], got[bad][:8], want[bad][:8])]
+
+
 @pytest.mark.parametrize("D,B,S", [(128, 2, 40), (128, 3, 1), (40, 1, 700), (8, 2, 3)])
 def test_rope_by_token_is_the_transposed_form(cuda, D, B, S):
     nh, nkv, cur, T = 6, 2, 3, S + 5
