@@ -379,7 +379,7 @@ def run_ours(args, world, rank, local, dist):
                                  "peak_src": peaks["src"], "unit": "GB/s", "frac": b * steps / t / 1e9 / peaks["hbm_gbs"], "traffic": None})
         out.update(ms_per_step=t / steps * 1e3, clocks=cs.summary(), gpu_launches=steps,
                    config={"workload": f"int4 GEMM + {'per-token asymmetric x per-channel' if asym else 'group-128'} dequant, M={M}, {K}->{N}, f16 out",
-                           "M": M, "N": N, "K": K, "algo": int(_lib.load().flh_b200_gemm_pick_algo(M, N, K, K if asym else 128, K if asym else 128)),
+                           "M": M, "N": N, "K": K, "algo": int(_algo(M, N, K, K if asym else 128)),
                            "weights_prepacked_int8": prepack,
                            "l2": "weights of three rotating problems (3 x 45 MB > L2); the K steps run as one CUDA graph" if not prefill else "operands re-used across steps (compute-bound)",
                            "parallelism": f"replicated x{world}, no collective"})
@@ -718,8 +718,15 @@ def grid_tables(C, device, peaks):
 
 
 def _algo(m, n, k, group):
-    from flh_b200 import _lib
-    return _lib.load().flh_b200_gemm_pick_algo(m, n, k, group, group)
+    """The kernel that gemm_i4_dequant runs: the one AUTO names, or one of the two it takes instead."""
+    from flh_b200 import _CUDA, _lib
+    lib = _lib.load()
+    picked, need = lib.flh_b200_gemm_pick_algo(m, n, k, group, group), lib.flh_b200_gemm_workspace_bytes(m, n, k, group, group, _CUDA.GEMM_AUTO_WORKSPACE)
+    if m <= 64 and need == 0 and (picked in (_CUDA.GEMM_STREAM_SPLITK, _CUDA.GEMM_DECODE_TC) or (group == k and m <= 32)):
+        return _CUDA.GEMM_DECODE_RING
+    if need and picked == _CUDA.GEMM_TCGEN05:
+        return _CUDA.GEMM_GROUP_F8
+    return picked
 
 
 def extras(C, device, peaks):

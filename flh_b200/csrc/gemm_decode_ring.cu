@@ -123,8 +123,9 @@ gemm_decode_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         if (lane == 0) {
             int it = 0;
             bool ok = true;
-            // while the kernel that makes the tokens still runs, the first stages of weights come into the L2 cache (a prefetch
-            // reads no value, so it needs no order with whatever wrote them)
+            // With group scales the first stages of weights come into the L2 cache while the kernel that makes the tokens still runs
+            // (a prefetch reads no value, so it needs no order with whatever wrote them).  Without them the barrier above waits
+            // for the threads that fetch the token scales behind their own wait, and the prefetch overlaps nothing.
             for (int st = 0; st < S && st < p.steps && (int)blockIdx.x < p.tiles; ++st)
 #pragma unroll
                 for (int k = 0; k < WK; ++k) tma_prefetch_2d(&map_w, (st * WK + k) * 128, blockIdx.x * BR);

@@ -75,19 +75,19 @@ __global__ void __launch_bounds__(256) prep_group_f8_kernel(const PrepParams p) 
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-        const long i = i0 + u * stride;
-        if (i >= total) break;
-        const bool isb = i >= p.a16;
-        const long j = isb ? i - p.a16 : i;
-        const uint4 w = wv[u];
-        uint4 e, o;
-        e.x = nibbles_to_f8(w.x & 0x0F0F0F0Fu); e.y = nibbles_to_f8(w.y & 0x0F0F0F0Fu);
-        e.z = nibbles_to_f8(w.z & 0x0F0F0F0Fu); e.w = nibbles_to_f8(w.w & 0x0F0F0F0Fu);
-        o.x = nibbles_to_f8((w.x >> 4) & 0x0F0F0F0Fu); o.y = nibbles_to_f8((w.y >> 4) & 0x0F0F0F0Fu);
-        o.z = nibbles_to_f8((w.z >> 4) & 0x0F0F0F0Fu); o.w = nibbles_to_f8((w.w >> 4) & 0x0F0F0F0Fu);
-        uint4 *out = (isb ? p.eb : p.ea) + 2 * j;
-        out[0] = e;
-        out[1] = o;
+            const long i = i0 + u * stride;
+            if (i >= total) break;
+            const bool isb = i >= p.a16;
+            const long j = isb ? i - p.a16 : i;
+            const uint4 w = wv[u];
+            uint4 e, o;
+            e.x = nibbles_to_f8(w.x & 0x0F0F0F0Fu); e.y = nibbles_to_f8(w.y & 0x0F0F0F0Fu);
+            e.z = nibbles_to_f8(w.z & 0x0F0F0F0Fu); e.w = nibbles_to_f8(w.w & 0x0F0F0F0Fu);
+            o.x = nibbles_to_f8((w.x >> 4) & 0x0F0F0F0Fu); o.y = nibbles_to_f8((w.y >> 4) & 0x0F0F0F0Fu);
+            o.z = nibbles_to_f8((w.z >> 4) & 0x0F0F0F0Fu); o.w = nibbles_to_f8((w.w >> 4) & 0x0F0F0F0Fu);
+            uint4 *out = (isb ? p.eb : p.ea) + 2 * j;
+            out[0] = e;
+            out[1] = o;
         }
     }
     // scales: a thread takes one row and eight consecutive groups, so that its 2-byte reads share a sector

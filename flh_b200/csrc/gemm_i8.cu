@@ -58,15 +58,15 @@ __global__ void __launch_bounds__(256) expand_i4_kernel(const uint4 *__restrict_
             if (i0 + u * stride < n16) wv[u] = ldg_nc_v4(in + i0 + u * stride);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-        const long i = i0 + u * stride;
-        if (i >= n16) break;
-        const uint4 w = wv[u];
-        uint4 e, o;
-        e.x = (w.x << 4) & 0xF0F0F0F0u; e.y = (w.y << 4) & 0xF0F0F0F0u;
-        e.z = (w.z << 4) & 0xF0F0F0F0u; e.w = (w.w << 4) & 0xF0F0F0F0u;
-        o.x = w.x & 0xF0F0F0F0u; o.y = w.y & 0xF0F0F0F0u; o.z = w.z & 0xF0F0F0F0u; o.w = w.w & 0xF0F0F0F0u;
-        out[2 * i] = e;
-        out[2 * i + 1] = o;
+            const long i = i0 + u * stride;
+            if (i >= n16) break;
+            const uint4 w = wv[u];
+            uint4 e, o;
+            e.x = (w.x << 4) & 0xF0F0F0F0u; e.y = (w.y << 4) & 0xF0F0F0F0u;
+            e.z = (w.z << 4) & 0xF0F0F0F0u; e.w = (w.w << 4) & 0xF0F0F0F0u;
+            o.x = w.x & 0xF0F0F0F0u; o.y = w.y & 0xF0F0F0F0u; o.z = w.z & 0xF0F0F0F0u; o.w = w.w & 0xF0F0F0F0u;
+            out[2 * i] = e;
+            out[2 * i + 1] = o;
         }
     }
 }

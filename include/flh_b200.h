@@ -263,7 +263,8 @@ int flh_b200_gptq_block(const float *W, long ldw, const float *Hinv, long ldh, c
                         long lds, const int *group_of_col, long rows, int count, int maxq, int sym, float clip_ratio,
                         float *Q, long ldq, float *Err, void *stream);
 
-/* Which algorithm FLH_B200_GEMM_AUTO resolves to for this shape (one of FLH_B200_GEMM_*). */
+/* Which algorithm FLH_B200_GEMM_AUTO resolves to for this shape (one of FLH_B200_GEMM_*), given its workspace, where neither
+ * DECODE_RING nor GROUP_F8 takes the call in its place (see their definitions). */
 int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group);
 
 /* Decode GEMM (M <= 64) for callers that must not allocate.  Same arguments and results as
