@@ -13,8 +13,9 @@
 // block instead of 96.  Per block the MMA thread fills one of two TMEM buffers while the epilogue warps fold the other.
 //
 // Measured (B200, expansion included): 2048 x 4096 -> 12288 179 us, 8192 -> 57344 1,395 us, 11008 -> 4096 159 us; the converting
-// kernel of gemm_tcgen05.cu, which has the same results, 266, 2,399 and 247 us.  A block takes about 1,300 clocks: the epilogue
-// 1,030 of them, then about 300 until it sees the next accumulator.
+// kernel of gemm_tcgen05.cu, which has the same results, 266, 2,399 and 247 us.  A block takes 1,410 clocks (the slope over K of a launch
+// of one tile per pair; 1,030 of them the fold, timed inside an instrumented copy of the loop, the rest until the epilogue sees the
+// next accumulator), the fill and the store of a tile another 5,600: 305,000 clocks for the six waves of 2048 x 4096 -> 12288.
 //
 //   warp 0   TMA: 128 rows of A and BN / 2 rows of B per stage        warp 1   MMA issuer (the leader's)
 //   warp 2   bulk copies of a block's scales                          warps 4-11 epilogue, 32 rows x BN / 2 columns each
