@@ -99,4 +99,11 @@ __device__ __forceinline__ uint4 ldg_v4(const void *p) {
     return v;
 }
 
+// 32 bytes of one thread to a 32-byte aligned address, as one store: a whole sector, where two 16-byte stores of a warp that
+// leaves gaps between its lanes are two half-written ones each
+__device__ __forceinline__ void stg_v8(void *p, const uint4 a, const uint4 b) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+}
+
 }  // namespace flh

@@ -12,13 +12,13 @@
 // A pair of CTAs (cta_group::2) shares one 256 x BN tile, as in gemm_i8.cu: 64 KB of shared-memory traffic per CTA and
 // block instead of 96.  Per block the MMA thread fills one of two TMEM buffers while the epilogue warps fold the other.
 //
-// Measured (B200, expansion included): 2048 x 4096 -> 12288 179 us, 8192 -> 57344 1,395 us, 11008 -> 4096 159 us; the converting
-// kernel of gemm_tcgen05.cu, which has the same results, 266, 2,399 and 247 us.  A block takes 1,410 clocks (the slope over K of a launch
-// of one tile per pair; 1,030 of them the fold, timed inside an instrumented copy of the loop, the rest until the epilogue sees the
-// next accumulator), the fill and the store of a tile another 5,600: 305,000 clocks for the six waves of 2048 x 4096 -> 12288.
+// Measured (B200, expansion included): 2048 x 4096 -> 12288 179 us, 4096 -> 22016 292 us, 11008 -> 4096 161 us (with eight epilogue
+// warps, one-lane issue loops and 16-byte stores in the expansion 183, 298 and 163); the converting kernel of gemm_tcgen05.cu, which
+// has the same results, 266, 439 and 247 us.  Of the 179 us 93 remain without any work in the epilogue and 110 with its TMEM loads
+// only: the epilogue is the limit.
 //
 //   warp 0   TMA: 128 rows of A and BN / 2 rows of B per stage        warp 1   MMA issuer (the leader's)
-//   warp 2   bulk copies of a block's scales                          warps 4-11 epilogue, 32 rows x BN / 2 columns each
+//   warp 2   bulk copies of a block's scales                          warps 4-19 epilogue, 32 rows x 64 columns each
 //
 // Every wait is bounded (two seconds) and reports through a status word, as in the other GEMM kernels.
 #include "tc_common.cuh"
@@ -30,7 +30,8 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 128;                  // K of a block = one group = one 128-byte swizzle row of e4m3
 constexpr int kRing = 8;                 // scale slots
-constexpr int EW = 8;                    // epilogue warps
+constexpr int EW = 16;                   // epilogue warps, 32 rows x 64 columns each
+constexpr int BN = 256;                  // columns of a tile
 
 __device__ int g_status_f8[4];
 
@@ -53,6 +54,10 @@ __device__ __forceinline__ uint32_t nibbles_to_f8(uint32_t x) {
     const uint32_t s = x & 0x08080808u, one = s >> 3;
     return ((((x & 0x07070707u) ^ (s - one)) + one)) | (s << 4);
 }
+// Where the scale of a row or column lies within its group's line: so that what one epilogue thread needs is 16 bytes.  It holds
+// rows r, r + 8, r + 16, r + 24 of 32 and, of every 16 columns, 2 q, 2 q + 1, 8 + 2 q and 9 + 2 q.
+__device__ __forceinline__ int row_slot(int r) { return (r & ~31) | ((r & 7) << 2) | ((r >> 3) & 3); }
+__device__ __forceinline__ int col_slot(int c) { return (c & ~15) | ((c & 6) << 1) | ((c >> 2) & 2) | (c & 1); }
 // bound by memory: 1.5 bytes per code of A and B; the scales are a few per cent of that
 struct PrepParams {
     const uint4 *a, *b;
@@ -86,9 +91,7 @@ __global__ void __launch_bounds__(256) prep_group_f8_kernel(const PrepParams p) 
             e.z = nibbles_to_f8(w.z & 0x0F0F0F0Fu); e.w = nibbles_to_f8(w.w & 0x0F0F0F0Fu);
             o.x = nibbles_to_f8((w.x >> 4) & 0x0F0F0F0Fu); o.y = nibbles_to_f8((w.y >> 4) & 0x0F0F0F0Fu);
             o.z = nibbles_to_f8((w.z >> 4) & 0x0F0F0F0Fu); o.w = nibbles_to_f8((w.w >> 4) & 0x0F0F0F0Fu);
-            uint4 *out = (isb ? p.eb : p.ea) + 2 * j;
-            out[0] = e;
-            out[1] = o;
+            stg_v8((isb ? p.eb : p.ea) + 2 * j, e, o);
         }
     }
     // scales: a thread takes one row and eight consecutive groups, so that its 2-byte reads share a sector
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(256) prep_group_f8_kernel(const PrepParams p) 
         const int g0 = (int)(j / rows) * 8, r = (int)(j - (long)(j / rows) * rows);
         const int cols = isb ? p.gb_cols : p.ga_cols;
         const __half *src = (isb ? p.b_scale : p.a_scale) + (long)r * cols;
-        float *dst = (isb ? p.sb : p.sa) + r;
+        float *dst = (isb ? p.sb : p.sa) + (isb ? col_slot(r) : row_slot(r));
         const bool live = isb || r < p.M;
         const float unit = isb ? 1.0f : 262144.0f;       // the 2^18 of the two e4m3 operands
 #pragma unroll
@@ -120,7 +123,6 @@ struct F8Params {
     int num_tiles, m_blocks;             // tiles of 256 x BN, row blocks fastest
 };
 
-template <int BN>
 struct F8Plan {
     static constexpr int kStageBytes = (BM + BN / 2) * BK;
     static constexpr int kStages = 6;
@@ -131,11 +133,10 @@ struct F8Plan {
     static constexpr int kThreads = 128 + 32 * EW;
 };
 
-template <int BN>
-__global__ void __launch_bounds__(128 + 32 * EW, 1)
+__global__ void __launch_bounds__(F8Plan::kThreads, 1)
 gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const F8Params p) {
-    using Plan = F8Plan<BN>;
-    constexpr int S = Plan::kStages, COLS = BN * 4 / EW;    // COLS: columns of an epilogue warp
+    using Plan = F8Plan;
+    constexpr int S = Plan::kStages, COLS = 64;             // COLS: columns of an epilogue warp
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t raw = smem_u32(smem_dyn);
     const uint32_t base = (raw + 1023u) & ~1023u;         // the same offset in both CTAs of a pair
@@ -148,8 +149,8 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     auto sempty = [&](int s) { return bars + 8u * (24 + s); };
     auto acc_full = [&](int b) { return bars + 8u * (32 + b); };
     auto acc_empty = [&](int b) { return bars + 8u * (34 + b); };      // leader only
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + Plan::kBarOff + 8 * 36);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Plan::kBarOff + 8 * 36 + 8);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + Plan::kBarOff + 8 * 40);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Plan::kBarOff + 8 * 40 + 8);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int KB = p.KB;
@@ -175,27 +176,32 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const uint32_t tmem = *tmem_slot;
 
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::);     // 128 x 72 + 256 x 216 = 384 x 168, what the block is launched with
-        if (warp == 0 && lane == 0) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;" ::);     // 128 x 32 + 512 x 112 = 640 x 96, what the block is launched with
+        if (warp == 0) {
             // -------------------------------------------------------- TMA producer (own halves)
             pdl_wait();                      // the operands are made by the kernel before; the set-up above overlapped it
-            int it = 0;
+            int it = 0, s = 0;
+            uint32_t ph = 1;
             bool ok = true;
-            for (int tile = first; tile < p.num_tiles && ok; tile += step) {
+            for (int tile = first; tile < p.num_tiles; tile += step) {
                 const int m0 = (tile % p.m_blocks) * 2 * BM + (int)rank * BM;
                 const int n0 = (tile / p.m_blocks) * BN + (int)rank * (BN / 2);
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % S;
-                    if (!wait_f8(empty(s), ((it / S) & 1) ^ 1, abort_flag, 41)) { ok = false; break; }
+                for (int kb = 0; kb < KB; ++kb) {
+                    ok = __all_sync(0xffffffffu, ok && wait_f8(empty(s), ph, abort_flag, 41));
                     const uint32_t dst = base + s * Plan::kStageBytes;
-                    if (rank == 1) {
-                        tma_load_2d_to_leader(dst, &map_a, kb * BK, m0, full(s));
-                        tma_load_2d_to_leader(dst + BM * BK, &map_b, kb * BK, n0, full(s));
-                    } else {
-                        mbar_expect_tx(full(s), 2 * Plan::kStageBytes);
-                        tma_load_2d(dst, &map_a, kb * BK, m0, full(s));
-                        tma_load_2d(dst + BM * BK, &map_b, kb * BK, n0, full(s));
+                    if (ok && elect_one()) {
+                        if (rank == 1) {
+                            tma_load_2d_to_leader(dst, &map_a, kb * BK, m0, full(s));
+                            tma_load_2d_to_leader(dst + BM * BK, &map_b, kb * BK, n0, full(s));
+                        } else {
+                            mbar_expect_tx(full(s), 2 * Plan::kStageBytes);
+                            tma_load_2d(dst, &map_a, kb * BK, m0, full(s));
+                            tma_load_2d(dst + BM * BK, &map_b, kb * BK, n0, full(s));
+                        }
                     }
+                    __syncwarp();
+                    it += ok;
+                    if (++s == S) { s = 0; ph ^= 1; }
                 }
             }
             if (*abort_flag && rank == 0) {      // let the copies already issued land before the CTA leaves
@@ -204,44 +210,25 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     while (!mbar_try(full(j % S), (j / S) & 1) && gtimer() - t0 < 100000000ull) {}
                 }
             }
-        } else if (warp == 1 && lane == 0 && rank == 0) {
-            // -------------------------------------------------------- MMA issuer
-            // D binary32, A and B e4m3 (format 0), N = BN, M = 256
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-            int it = 0;
-            bool ok = true;
-            for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % S, buf = it & 1;
-                    // the operands are there long before; the buffer is what this thread waits for, and what the epilogue waits for
-                    // is the first thing it commits
-                    if (!wait_f8(full(s), (it / S) & 1, abort_flag, 43)) { ok = false; break; }
-                    if (it >= 2 && !wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_addr = base + s * Plan::kStageBytes;
-                    const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BM * BK);
-#pragma unroll
-                    for (int k4 = 0; k4 < BK / 32; ++k4)
-                        mma_f8_pair(tmem + buf * 256, adesc + 2 * k4, bdesc + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
-                    tc_commit_pair(acc_full(buf));
-                    tc_commit_pair(empty(s));
-                }
-            }
-        } else if (warp == 2 && lane == 0) {
+        } else if (warp == 2) {
             // -------------------------------------------------------- scales of every block
             pdl_wait();
-            int it = 0;
+            int it = 0, slot = 0;
+            uint32_t ph = 1;
             bool ok = true;
-            for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-                const int m0 = (tile % p.m_blocks) * 2 * BM + (int)rank * BM;
-                const int n0 = (tile / p.m_blocks) * BN;
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % kRing;
-                    if (!wait_f8(sempty(s), ((it / kRing) & 1) ^ 1, abort_flag, 44)) { ok = false; break; }
-                    const uint32_t dst = base + Plan::kRingOff + s * Plan::kSlot;
-                    mbar_expect_tx(sfull(s), Plan::kSlot);
-                    bulk_load(dst, p.sb + (long)kb * p.N + n0, BN * 4, sfull(s));
-                    bulk_load(dst + BN * 4, p.sa + (long)kb * p.Mp + m0, BM * 4, sfull(s));
+            for (int tile = first; tile < p.num_tiles; tile += step) {
+                const float *sa = p.sa + (tile % p.m_blocks) * 2 * BM + (int)rank * BM, *sb = p.sb + (tile / p.m_blocks) * BN;
+                for (int kb = 0; kb < KB; ++kb, sa += p.Mp, sb += p.N) {
+                    ok = __all_sync(0xffffffffu, ok && wait_f8(sempty(slot), ph, abort_flag, 44));
+                    const uint32_t dst = base + Plan::kRingOff + slot * Plan::kSlot;
+                    if (ok && elect_one()) {
+                        mbar_expect_tx(sfull(slot), Plan::kSlot);
+                        bulk_load(dst, sb, BN * 4, sfull(slot));
+                        bulk_load(dst + BN * 4, sa, BM * 4, sfull(slot));
+                    }
+                    __syncwarp();
+                    it += ok;
+                    if (++slot == kRing) { slot = 0; ph ^= 1; }
                 }
             }
             if (*abort_flag) {
@@ -250,10 +237,36 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     while (!mbar_try(sfull(j % kRing), (j / kRing) & 1) && gtimer() - t0 < 100000000ull) {}
                 }
             }
+        } else if (warp == 1 && rank == 0) {
+            // -------------------------------------------------------- MMA issuer (the whole warp walks the loop, see elect_one)
+            // D binary32, A and B e4m3 (format 0), N = BN, M = 256
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+            int it = 0, s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = first; tile < p.num_tiles; tile += step) {
+                for (int kb = 0; kb < KB; ++kb, ++it) {
+                    const int buf = it & 1;
+                    ok = __all_sync(0xffffffffu, ok && wait_f8(full(s), ph, abort_flag, 43) &&
+                                                     wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42));
+                    tc_fence_after();
+                    const uint32_t a_addr = base + s * Plan::kStageBytes;
+                    const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BM * BK);
+                    if (ok && elect_one()) {
+#pragma unroll
+                        for (int k4 = 0; k4 < BK / 32; ++k4)
+                            mma_f8_pair(tmem + buf * 256, adesc + 2 * k4, bdesc + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+                        tc_commit_pair(acc_full(buf));
+                        tc_commit_pair(empty(s));
+                    }
+                    __syncwarp();
+                    if (++s == S) { s = 0; ph ^= 1; }
+                }
+            }
         }
     } else {
         // ------------------------------------------------------------ epilogue
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;" ::);
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;" ::);
         const int wq = warp & 3;                         // TMEM lane quarter this warp may read
         const int c0 = ((warp - 4) >> 2) * COLS;         // first tile column of this warp
         const uint32_t tlane = tmem + ((uint32_t)(wq * 32) << 16) + c0;
@@ -282,31 +295,30 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 };
                 if (ok) {
                     const float *sl = reinterpret_cast<const float *>(sm + Plan::kRingOff + slot * Plan::kSlot);
-                    uint64_t sa2[4];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) { const float sa = sl[BN + r0 + 8 * r]; sa2[r] = pack2(sa, sa); }
-                    const uint64_t *sb = reinterpret_cast<const uint64_t *>(sl + c0) + (lane & 3);
                     const uint32_t src = tlane + buf * 256;
                     tc_fence_after();
-                    // the next 32 columns are on their way from TMEM while these are folded
-                    uint32_t vv[2][32];
-                    tc_ld_frag(src, vv[0]);
-                    tc_ld_frag(src + (16u << 16), vv[0] + 16);
+                    // the next 16 columns are on their way from TMEM while these are folded
+                    uint32_t vv[2][16];
+                    tc_ld_frag2(src, vv[0]);
+                    tc_ld_frag2(src + (16u << 16), vv[0] + 8);
+                    const float4 sa = *reinterpret_cast<const float4 *>(sl + BN + wq * 32 + (lane >> 2) * 4);
+                    const uint64_t sa2[4] = {pack2(sa.x, sa.x), pack2(sa.y, sa.y), pack2(sa.z, sa.z), pack2(sa.w, sa.w)};
+                    const ulonglong2 *sb = reinterpret_cast<const ulonglong2 *>(sl + c0) + (lane & 3);
 #pragma unroll
-                    for (int cc = 0; cc < COLS / 32; ++cc) {
+                    for (int cc = 0; cc < COLS / 16; ++cc) {
+                        const ulonglong2 sb2 = sb[cc * 4];
                         tc_wait_ld();
-                        if (cc + 1 < COLS / 32) {
-                            tc_ld_frag(src + (cc + 1) * 32, vv[(cc + 1) & 1]);
-                            tc_ld_frag(src + (cc + 1) * 32 + (16u << 16), vv[(cc + 1) & 1] + 16);
+                        if (cc + 1 < COLS / 16) {
+                            tc_ld_frag2(src + (cc + 1) * 16, vv[(cc + 1) & 1]);
+                            tc_ld_frag2(src + (cc + 1) * 16 + (16u << 16), vv[(cc + 1) & 1] + 8);
                         } else release_acc();
-                        const uint32_t (&v)[32] = vv[cc & 1];
+                        const uint32_t (&v)[16] = vv[cc & 1];
 #pragma unroll
-                        for (int n = 0; n < 4; ++n) {
-                            const uint64_t sb2 = sb[(cc * 4 + n) * 4];
+                        for (int n = 0; n < 2; ++n) {
 #pragma unroll
                             for (int r = 0; r < 4; ++r) {
-                                const int i = (r >> 1) * 16 + 4 * n + 2 * (r & 1);
-                                acc[r][cc * 4 + n] = fma2(((uint64_t)v[i + 1] << 32) | v[i], mul2(sa2[r], sb2), acc[r][cc * 4 + n]);
+                                const int i = (r >> 1) * 8 + 4 * n + 2 * (r & 1);
+                                acc[r][cc * 2 + n] = fma2(((uint64_t)v[i + 1] << 32) | v[i], mul2(sa2[r], n ? sb2.y : sb2.x), acc[r][cc * 2 + n]);
                             }
                         }
                     }
@@ -356,10 +368,9 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
 }
 
-template <int BN>
 int launch_f8(const CUtensorMap &ma, const CUtensorMap &mb, F8Params p, cudaStream_t stream) {
-    using Plan = F8Plan<BN>;
-    auto kern = gemm_group_f8_kernel<BN>;
+    using Plan = F8Plan;
+    auto kern = gemm_group_f8_kernel;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::kBytes);
     if (e != cudaSuccess) return cuda_status(e, "gemm_group_f8 attribute");
     p.m_blocks = (p.M + 2 * BM - 1) / (2 * BM);
@@ -428,7 +439,7 @@ int launch_gemm_group_f8(const uint8_t *A, const uint8_t *B, const void *a_scale
     if (rc) return rc;
     rc = make_map_bytes(&mb, eb, N, K, 128);
     if (rc) return rc;
-    return launch_f8<256>(ma, mb, p, stream);
+    return launch_f8(ma, mb, p, stream);
 }
 
 int gemm_group_f8_status(int *out4) {

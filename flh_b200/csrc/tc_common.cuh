@@ -22,6 +22,13 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// the state of the phase, without any wait in hardware
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 // try_wait with a suspend-time hint: the thread may sleep in hardware for up to `ns` nanoseconds instead of coming back at
 // once, so a waiting warp does not spend issue slots on a spin loop beside the warps that have work
 __device__ __forceinline__ bool mbar_try_hint(uint32_t bar, uint32_t parity, uint32_t ns) {
@@ -53,6 +60,15 @@ __device__ __forceinline__ bool mbar_wait_status(int *status, uint32_t bar, uint
             return false;
         }
     }
+}
+// One lane of a converged warp.  A loop that issues tcgen05 or TMA instructions is walked by its whole warp, and only the instructions
+// themselves are under this predicate: their operands are uniform registers, and in a loop that one lane walks (if (lane == 0)) each is
+// moved there again with the warp's divergence to manage.  Measured for an iteration of two waits, four MMAs and two commits: 596 clocks
+// by one lane, 377 - 409 so.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -88,6 +104,11 @@ __device__ __forceinline__ void tc_ld_frag(uint32_t taddr, uint32_t *v) {
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
                    "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                  : "r"(taddr) : "memory");
+}
+// the same, 16 lanes x 16 columns
+__device__ __forceinline__ void tc_ld_frag2(uint32_t taddr, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void bar_sync_named(int id, int nthreads) {
