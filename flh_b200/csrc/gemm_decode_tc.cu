@@ -2,9 +2,9 @@
 // weight tile are the M side of tcgen05.mma kind::i8 (one TMEM lane each), the tokens the N side (16, 32 or 64
 // columns), so the kernel streams the packed weights once and spends no CUDA-core multiply on them.
 //
-//   warp 0 (one thread)   TMA: 128 x 64 B of packed weights + TOK x 64 B of packed tokens per 128-K block -> smem ring
+//   warp 0                TMA: 128 x 64 B of packed weights + TOK x 64 B of packed tokens per 128-K block -> smem ring
 //   warps 2-5             nibbles -> int8 (x16) in the K-major 128-byte-swizzled layout tcgen05 reads
-//   warp 1 (one thread)   four tcgen05.mma (K = 32 each) per block; D[channel][token] int32 in TMEM
+//   warp 1                four tcgen05.mma (K = 32 each) per block; D[channel][token] int32 in TMEM
 //   warps 6-9 (6-13 for 64 tokens: two groups, 32 token columns each)
 //                         thread = output channel: tcgen05.ld of its token sums of a block, dequantise
 //                         (acc = fmaf(float(I_g), sa * sb, acc) per 128-K group, or once per channel), store D^T
@@ -41,7 +41,8 @@ __device__ unsigned long long g_wait_ns[8];
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code,
                                           unsigned long long *waited = nullptr) {
-    // the first try may already sleep in hardware, so the whole call is timed
+    // a try may already sleep in hardware, so what does not succeed at once is timed as a whole
+    if (mbar_test(bar, parity)) return true;
     const uint64_t t0 = waited ? gtimer() : 0;
     const bool ok = mbar_wait_status(g_status, bar, parity, abort_flag, code);
     if (waited) *waited += gtimer() - t0;
@@ -126,9 +127,9 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     int *za_s = reinterpret_cast<int *>(sa_s + sa_n);
 
     if (tid == 0) {
-        for (int s = 0; s < SP; ++s) { mbar_init(pk_full(s), 1); mbar_init(pk_empty(s), 128); }
-        for (int s = 0; s < SE; ++s) { mbar_init(ex_full(s), 128); mbar_init(ex_empty(s), 1); }
-        for (int b = 0; b < NBUF; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128 * EG); }
+        for (int s = 0; s < SP; ++s) { mbar_init(pk_full(s), 1); mbar_init(pk_empty(s), 4); }
+        for (int s = 0; s < SE; ++s) { mbar_init(ex_full(s), 4); mbar_init(ex_empty(s), 1); }
+        for (int b = 0; b < NBUF; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4 * EG); }
         *abort_flag = 0;
         s_last[0] = 0; s_last[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -146,61 +147,64 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            int tile = lin_begin / KB, kb = lin_begin - tile * KB;
-            int it = 0;
-            unsigned long long w1 = 0;
-            for (; it < count; ++it) {
-                const int s = it % SP;
-                if (!mbar_wait(pk_empty(s), ((it / SP) & 1) ^ 1, abort_flag, 1, &w1)) break;
+        int tile = lin_begin / KB, kb = lin_begin - tile * KB;
+        int it = 0, s = 0;
+        uint32_t ph = 1;
+        unsigned long long w1 = 0;
+        for (; it < count; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(pk_empty(s), ph, abort_flag, 1, &w1))) break;
+            const uint32_t dst = base + Plan::kPkOff + s * Plan::kPkStage;
+            if (elect_one()) {
                 mbar_expect_tx(pk_full(s), Plan::kPkStage);
-                const uint32_t dst = base + Plan::kPkOff + s * Plan::kPkStage;
                 tma_load_2d(dst, &map_w, kb * (BK / 2), tile * BR, pk_full(s));
                 tma_load_2d(dst + BR * (BK / 2), &map_x, kb * (BK / 2), 0, pk_full(s));
-                if (++kb == KB) { kb = 0; ++tile; }
             }
-            atomicAdd(&g_wait_ns[1], w1);
-            if (*abort_flag) {
-                // let the copies already issued land before the CTA leaves
-                for (int j = it > SP ? it - SP : 0; j < it; ++j) {
-                    const uint64_t t0 = gtimer();
-                    while (!mbar_try(pk_full(j % SP), (j / SP) & 1) && gtimer() - t0 < 100000000ull) {}
-                }
+            __syncwarp();
+            if (++kb == KB) { kb = 0; ++tile; }
+            if (++s == SP) { s = 0; ph ^= 1; }
+        }
+        if (lane == 0) atomicAdd(&g_wait_ns[1], w1);
+        if (*abort_flag) {
+            // let the copies already issued land before the CTA leaves
+            for (int j = it > SP ? it - SP : 0; j < it; ++j) {
+                const uint64_t t0 = gtimer();
+                while (!mbar_try(pk_full(j % SP), (j / SP) & 1) && gtimer() - t0 < 100000000ull) {}
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            // D s32; A = weights (signed), B = tokens (unsigned codes with zero-points, else signed); N = TOK, M = 128
-            const uint32_t idesc = (2u << 4) | (1u << 7) | ((A_UNSIGNED ? 0u : 1u) << 10) |
-                                   ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(BR >> 4) << 24);
-            int kb = lin_begin % KB;
-            int u = 0;
-            unsigned long long w2 = 0, w3 = 0;
-            for (int it = 0; it < count; ++it) {
-                const int s = it % SE;
-                const int buf = u % NBUF;
-                const bool seg_first = it == 0 || kb == 0;
-                const bool seg_last = it == count - 1 || kb == KB - 1;
-                if ((GROUPED || seg_first) && u >= NBUF) {
-                    if (!mbar_wait(acc_empty(buf), ((u / NBUF) & 1) ^ 1, abort_flag, 2, &w2)) break;
-                }
-                if (!mbar_wait(ex_full(s), (it / SE) & 1, abort_flag, 3, &w3)) break;
-                tc_fence_after();
-                const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage;
-                const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
+        // ------------------------------------------------------------ MMA issuer (the whole warp walks the loop, see elect_one)
+        // D s32; A = weights (signed), B = tokens (unsigned codes with zero-points, else signed); N = TOK, M = 128
+        const uint32_t idesc = (2u << 4) | (1u << 7) | ((A_UNSIGNED ? 0u : 1u) << 10) |
+                               ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(BR >> 4) << 24);
+        int kb = lin_begin % KB;
+        int u = 0, s = 0;
+        uint32_t ph = 0;
+        unsigned long long w2 = 0, w3 = 0;
+        for (int it = 0; it < count; ++it) {
+            const int buf = u % NBUF;
+            const bool seg_first = it == 0 || kb == 0;
+            const bool seg_last = it == count - 1 || kb == KB - 1;
+            bool ok = true;
+            if ((GROUPED || seg_first) && u >= NBUF) ok = mbar_wait(acc_empty(buf), ((u / NBUF) & 1) ^ 1, abort_flag, 2, &w2);
+            if (!__all_sync(0xffffffffu, ok && mbar_wait(ex_full(s), ph, abort_flag, 3, &w3))) break;
+            tc_fence_after();
+            const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage;
+            const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
+            if (elect_one()) {
 #pragma unroll
                 for (int k4 = 0; k4 < BK / 32; ++k4) {
                     const uint32_t accum = GROUPED ? (k4 > 0) : (!seg_first || k4 > 0);
                     tc_mma_i8(tmem + buf * TOK, adesc + 2 * k4, bdesc + 2 * k4, idesc, accum);
                 }
                 tc_commit(ex_empty(s));
-                if (GROUPED || seg_last) { tc_commit(acc_full(buf)); ++u; }
-                if (++kb == KB) kb = 0;
+                if (GROUPED || seg_last) tc_commit(acc_full(buf));
             }
-            atomicAdd(&g_wait_ns[2], w2);
-            atomicAdd(&g_wait_ns[3], w3);
+            __syncwarp();
+            if (GROUPED || seg_last) ++u;
+            if (++kb == KB) kb = 0;
+            if (++s == SE) { s = 0; ph ^= 1; }
         }
+        if (lane == 0) { atomicAdd(&g_wait_ns[2], w2); atomicAdd(&g_wait_ns[3], w3); }
     } else if (warp < 6) {
         // ------------------------------------------------------------ int4 -> int8 converters
         const int ct = tid - 64;                          // 0..127
@@ -217,8 +221,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         unsigned long long w4 = 0, w5 = 0;
         for (int it = 0; it < count; ++it) {
             const int sp = it % SP, se = it % SE;
-            if (!mbar_wait(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4)) break;
-            if (!mbar_wait(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4) &&
+                                             mbar_wait(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5))) break;
             const uint8_t *pk = sm + Plan::kPkOff + sp * Plan::kPkStage;
             uint8_t *ex = sm + Plan::kExOff + se * Plan::kExStage;
             uint4 wv[kPerT];
@@ -238,8 +242,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
             fence_proxy_async();
-            mbar_arrive(ex_full(se));
-            mbar_arrive(pk_empty(sp));
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(ex_full(se)); mbar_arrive(pk_empty(sp)); }
         }
         if (ct == 0) { atomicAdd(&g_wait_ns[4], w4); atomicAdd(&g_wait_ns[5], w5); }
     } else {
@@ -303,7 +307,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     uint32_t v[TE];
                     if (ok) { tmem_ld_cols<TE>(tlane + buf * TOK + j0, v); tc_wait_ld(); }
                     tc_fence_before();
-                    mbar_arrive(acc_empty(buf));
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty(buf));
                     if (ok) {
                         const float *sa = sa_s + gas * kb + j0;
                         const int *za = za_s + gas * kb + j0;
@@ -326,7 +331,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 uint32_t v[TE];
                 if (ok) { tmem_ld_cols<TE>(tlane + buf * TOK + j0, v); tc_wait_ld(); }
                 tc_fence_before();
-                mbar_arrive(acc_empty(buf));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(buf));
                 ++u;
 #pragma unroll
                 for (int j = 0; j < TE; ++j) acci[j] = ok ? (int)v[j] : 0;
