@@ -20,6 +20,10 @@ import torch
 
 from . import _lib
 from .hadamard import get_hadK
+try:
+    from . import _host         # csrc/host_calls.cpp: the same calls with less host time; built by `python -m flh_b200.build`
+except ImportError:             # not built yet, or a torch without CUDA
+    _host = None
 
 F16, BF16 = 0, 1
 GEMM_AUTO, GEMM_TCGEN05, GEMM_MMA_SYNC, GEMM_STREAM, GEMM_STREAM_SPLITK, GEMM_TCGEN05_DIRECT = 0, 1, 2, 3, 4, 5
@@ -117,6 +121,10 @@ def _launch_quant_group(x, rows, gs, hadamard, q, s):
 def act_quant_group(x, gs: int, hadamard: bool):
     """The group quantiser over the last dimension of x [.., K]: -> (q u8[.., K/2], scale f16[.., K/gs]), the scales those of the
     normalised transform (the kernel's is un-normalised)."""
+    if _host is not None:
+        r = _host.act_quant_group(x, gs, hadamard)
+        if r is not None:
+            return r
     lead, K = x.shape[:-1], x.shape[-1]
     _check(gs in (32, 64, 128), "group_size must be 32, 64, or 128")
     _check(K % gs == 0 or x.numel() == 0, "the last dimension must be a multiple of group_size")
@@ -239,6 +247,11 @@ def _launch_quant_token(x, M, K, ld, hadamard, clip, exact, q, s, z):
 def act_quant_token(x, hadamard: bool, clip: float):
     """quant_token_asym_i4 over the last dimension of x [.., K]: -> (q u8[.., K/2], scale f16[.., 1], zero f16[.., 1])."""
     lead, K = x.shape[:-1], x.shape[-1]
+    if _host is not None and x.is_cuda and x.dtype in (torch.float16, torch.bfloat16):
+        kfac, bits = _sign_bits(K, x.device) if hadamard else (1, None)
+        r = _host.act_quant_token(x, hadamard, clip, kfac, bits)
+        if r is not None:
+            return r
     if not x.is_contiguous() or x.numel() == 0:
         q, s, z = quant_token_asym_i4(x.reshape(-1, K), hadamard=hadamard, clip=clip)
         return q.view(lead + (K // 2,)), s.view(lead + (1,)), z.view(lead + (1,))
@@ -427,6 +440,22 @@ def _launch_gemm(A, B, A_scale, A_zero, B_scale, B_rowsum, bias, D, M, N, K, ag,
             _ptr(A), _ptr(B), _ptr(A_scale), _ptr(A_zero), _ptr(B_scale), _ptr(B_rowsum), _ptr(bias), _ptr(D),
             M, N, K, ag, bg, BF16 if D.dtype == torch.bfloat16 else F16, algo, _ptr(ws), ws.numel() if ws is not None else 0,
             stream), "gemm_i4_dequant")
+
+
+def linear(x, w, a_scale, a_zero, w_scale, rowsum, bias, dtype):
+    """The GEMM of AUTO's choice for x [.., K/2] and packed weights w (flat or [N, K/2]) -> [.., N], through the native call; None
+    where that does not take the arguments (the caller goes through gemm_i4_dequant)."""
+    if _host is None or not x.is_cuda or dtype not in (torch.float16, torch.bfloat16) or x.numel() == 0 or a_scale.numel() == 0 or w_scale.dim() != 2:
+        return None
+    device, kp = x.device, x.shape[-1]
+    M, K, (N, gb) = x.numel() // kp, 2 * kp, w_scale.shape
+    ga = a_scale.numel() // M
+    if ga == 0 or gb == 0 or N == 0 or device.index != torch.cuda.current_device():
+        return None
+    words = (a_scale.data_ptr() | w_scale.data_ptr()) % 4 == 0
+    algo, need, zeroed = _gemm_plan(_lib.load(), M, N, K, K // ga, K // gb, GEMM_AUTO, a_zero is not None, words)
+    ws = None if not need else _workspace(device, _getrawstream(device.index), need) if zeroed else need
+    return _host.gemm(x, w, a_scale, a_zero, w_scale, rowsum, bias, dtype == torch.bfloat16, algo, ws)
 
 
 def expand_i4(B):

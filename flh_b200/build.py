@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SOURCES = ["api.cu", "quant_group.cu", "quant_token.cu", "quant_token_warp.cu", "quant_token_factor.cu", "quant_token_tc.cu", "act.cu", "gemm_mma.cu", "gemm_tcgen05.cu", "gemm_i8.cu", "gemm_group_f8.cu", "gemm_decode_tc.cu", "gemm_decode_ring.cu", "gptq.cu", "allreduce.cu"]
 LIB = os.path.join(HERE, "libflh_b200.so")
+HOST = os.path.join(HERE, "_host.so")             # csrc/host_calls.cpp: the per-call host work as a Python extension on torch
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
@@ -55,7 +56,24 @@ def build(verbose: bool = False, force: bool = False) -> str:
         list(ex.map(run, jobs))
     if force or jobs or not os.path.exists(LIB):
         run([nvcc, "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a"])
+    _build_host(run, force)
     return LIB
+
+
+def _build_host(run, force: bool) -> None:
+    src = os.path.join(CSRC, "host_calls.cpp")
+    if not force and not _stale(HOST, [src, os.path.join(HERE, "..", "include", "flh_b200.h")]):
+        return
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    if torch.version.cuda is None:
+        return                                      # nothing to launch on: flh_b200/_CUDA.py does without
+    include = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cpp_extension.CUDA_HOME or "/usr/local/cuda", "include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+         *[f"-I{i}" for i in include], src, "-o", HOST, f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_cuda",
+         "-ltorch_python", f"-L{HERE}", "-l:libflh_b200.so", "-Wl,-rpath,$ORIGIN"])
 
 
 if __name__ == "__main__":

@@ -1,0 +1,153 @@
+// The calls a decode step makes most — quantise the activations, multiply them with packed weights — without the Python around
+// them: argument checks, output allocation and the launch through the C ABI in one native function each.  What bounds the
+// smallest calls is the host: one token through a quantiser and a 4096 -> 12288 linear is 14 us of GPU work; through the Python of
+// flh_b200/_CUDA.py (checks, views, torch.empty, ctypes) it takes 35 us, so 17 (16 tokens through 11008 -> 4096: 42 and 21).
+//
+// Every function takes the plain case only and returns None for anything else — another type, layout or device than the
+// current one, a tensor subclass, a transform, mode or trace that has to see the operations — and the caller then goes the
+// way in Python, which has the error messages and the general shapes.  Nothing is kept between calls.
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <cmath>
+
+#include "../../include/flh_b200.h"
+
+namespace {
+
+// operations that something other than this process's kernels has to see
+bool observed() {
+    return at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() || torch::jit::tracer::isTracing();
+}
+// a contiguous CUDA tensor on `device` with memory of its own kind and nothing wrapped around it
+bool plain(const at::Tensor &t, c10::DeviceIndex device) {
+    if (!t.is_cuda() || t.device().index() != device || t.layout() != at::kStrided || !t.is_contiguous() || t.is_neg() || t.is_conj()) return false;
+    const c10::DispatchKeySet ks = t.key_set();
+    return !ks.has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchBatched,
+                                            c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched, c10::DispatchKey::ZeroTensor}));
+}
+const at::Tensor *tensor(PyObject *o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+PyObject *failed(const char *what, int rc) {
+    PyErr_Format(PyExc_RuntimeError, "%s failed (status %d): %s", what, rc, flh_b200_last_error());
+    return nullptr;
+}
+at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Tensor &like) {
+    return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+}
+// the sizes of x with the last one replaced
+c10::SmallVector<int64_t, 6> with_last(const at::Tensor &x, int64_t last) {
+    c10::SmallVector<int64_t, 6> s(x.sizes().begin(), x.sizes().end());
+    s.back() = last;
+    return s;
+}
+
+// act_quant_group(x, group_size, hadamard) -> (q, scale)
+PyObject *act_quant_group(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    const at::Tensor *x = n == 3 ? tensor(args[0]) : nullptr;
+    const long gs = x ? PyLong_AsLong(args[1]) : 0;
+    const int had = x ? PyObject_IsTrue(args[2]) : 0;
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    if (!x || observed() || (gs != 32 && gs != 64 && gs != 128) || x->dim() < 1 || x->scalar_type() != at::kHalf) Py_RETURN_NONE;
+    const c10::DeviceIndex dev = c10::cuda::current_device();
+    const int64_t K = x->size(-1);
+    if (!plain(*x, dev) || x->numel() == 0 || K % gs) Py_RETURN_NONE;
+    at::Tensor q = empty(with_last(*x, K / 2), at::kByte, *x), s = empty(with_last(*x, K / gs), at::kHalf, *x);
+    const int rc = flh_b200_quant_group_sym_i4(x->data_ptr(), x->numel() / gs, (int)gs, had, static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(),
+                                               c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc) return failed("quant_group_sym_i4", rc);
+    if (had) s = at::div(s, at::Scalar(std::sqrt((double)gs)));
+    return Py_BuildValue("(NN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)));
+    END_HANDLE_TH_ERRORS
+}
+
+// act_quant_token(x, hadamard, clip, kfac, sign table or None) -> (q, scale, zero)
+PyObject *act_quant_token(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    const at::Tensor *x = n == 5 ? tensor(args[0]) : nullptr;
+    const at::Tensor *bits = x ? tensor(args[4]) : nullptr;
+    const int had = x ? PyObject_IsTrue(args[1]) : 0;
+    const double clip = x ? PyFloat_AsDouble(args[2]) : 0;
+    const long kfac = x ? PyLong_AsLong(args[3]) : 0;
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    if (!x || (!bits && args[4] != Py_None) || observed() || x->dim() < 1) Py_RETURN_NONE;
+    if (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16) Py_RETURN_NONE;
+    const c10::DeviceIndex dev = c10::cuda::current_device();
+    if (!plain(*x, dev) || x->numel() == 0) Py_RETURN_NONE;
+    const int64_t K = x->size(-1);
+    const auto one = with_last(*x, 1);
+    at::Tensor q = empty(with_last(*x, K / 2), at::kByte, *x), s = empty(one, at::kHalf, *x), z = empty(one, at::kHalf, *x);
+    const int rc = flh_b200_quant_token_asym_i4(x->data_ptr(), x->scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, x->numel() / K, K, K,
+                                                had ? 1 : 0, (int)kfac, bits ? static_cast<const uint32_t *>(bits->data_ptr()) : nullptr, (float)clip,
+                                                static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(), z.data_ptr(),
+                                                c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc) return failed("quant_token_asym_i4", rc);
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)), THPVariable_Wrap(std::move(z)));
+    END_HANDLE_TH_ERRORS
+}
+
+// gemm(x, w, a_scale, a_zero, w_scale, rowsum, bias, bfloat16, algo, workspace) -> y: algo and workspace as the plan of
+// flh_b200/_CUDA.py names them, the workspace a tensor, the bytes of scratch that this call alone uses, or None.
+// x [.., K / 2], w flat or [N, K / 2].
+PyObject *gemm(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 10) Py_RETURN_NONE;
+    const at::Tensor *t[7];
+    for (int i = 0; i < 7; ++i) {
+        t[i] = tensor(args[i]);
+        if (!t[i] && (args[i] != Py_None || i < 3 || i == 4)) Py_RETURN_NONE;
+    }
+    const at::Tensor *ws = tensor(args[9]);
+    const long scratch = PyLong_Check(args[9]) ? PyLong_AsLong(args[9]) : 0;
+    const int bf16 = PyObject_IsTrue(args[7]);
+    const long algo = PyLong_AsLong(args[8]);
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    if ((!ws && !PyLong_Check(args[9]) && args[9] != Py_None) || observed()) Py_RETURN_NONE;
+    const at::Tensor &x = *t[0], &w = *t[1], &sa = *t[2], &sb = *t[4];
+    const c10::DeviceIndex dev = c10::cuda::current_device();
+    for (int i = 0; i < 7; ++i)
+        if (t[i] && !plain(*t[i], dev)) Py_RETURN_NONE;
+    if (x.dim() < 1 || sb.dim() != 2 || x.numel() == 0 || sb.numel() == 0) Py_RETURN_NONE;
+    const int64_t K = 2 * x.size(-1), M = x.numel() / x.size(-1), N = sb.size(0);
+    if (sa.numel() == 0 || sa.numel() % M || w.numel() != N * (K / 2)) Py_RETURN_NONE;
+    const int64_t ga = sa.numel() / M, gb = sb.size(1);
+    if (K % ga || K % gb || x.scalar_type() != at::kByte || w.scalar_type() != at::kByte || sa.scalar_type() != at::kHalf ||
+        sb.scalar_type() != at::kHalf || (t[3] && (t[3]->scalar_type() != at::kHalf || t[3]->numel() != sa.numel())) ||
+        (t[5] && t[5]->scalar_type() != at::kInt) || (t[6] && (t[6]->scalar_type() != at::kHalf || t[6]->numel() != N)))
+        Py_RETURN_NONE;
+    at::Tensor y = empty(with_last(x, N), bf16 ? at::kBFloat16 : at::kHalf, x), own;
+    if (scratch > 0) {
+        try {
+            own = empty({(int64_t)scratch}, at::kByte, x);       // freed in stream order when the call returns
+        } catch (const c10::OutOfMemoryError &) {
+            Py_RETURN_NONE;                                      // AUTO has a kernel that needs none
+        }
+        ws = &own;
+    }
+    const int rc = flh_b200_gemm_i4_dequant(
+        static_cast<const uint8_t *>(x.data_ptr()), static_cast<const uint8_t *>(w.data_ptr()), sa.data_ptr(), t[3] ? t[3]->data_ptr() : nullptr,
+        sb.data_ptr(), t[5] ? static_cast<const int32_t *>(t[5]->data_ptr()) : nullptr, t[6] ? t[6]->data_ptr() : nullptr, y.data_ptr(), M, N, K,
+        K / ga, K / gb, bf16 ? FLH_B200_BF16 : FLH_B200_F16, (int)algo, ws ? ws->data_ptr() : nullptr, ws ? (size_t)ws->numel() : 0,
+        c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc) return failed("gemm_i4_dequant", rc);
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"act_quant_group", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(act_quant_group)), METH_FASTCALL, nullptr},
+    {"act_quant_token", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(act_quant_token)), METH_FASTCALL, nullptr},
+    {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(gemm)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

@@ -262,6 +262,11 @@ class LinearFLH(torch.nn.Module):
         lead = x.shape[:-1]
         M = x.numel() // x.shape[-1]
         N, w_scale = self.out_features, self.w_scale
+        if out is None and M > 0 and x.shape[-1] * 2 == self.in_features and (self._w_i8 is None or M < self.PREPACK_MIN_ROWS):
+            rs = None if a_zero is None else self.w_rowsum(min(self.in_features // (a_scale.numel() // M or 1), self.in_features // w_scale.shape[1]))
+            y = _CUDA.linear(x, self.w_packed, a_scale, a_zero, w_scale, rs, self.bias, out_dtype or w_scale.dtype)
+            if y is not None:
+                return y
         if M == 0 or a_scale.dim() != 2 or a_scale.shape[0] != M or not a_scale.is_contiguous():
             a_scale = a_scale.reshape(M, -1)
         ga, gb = self.in_features // a_scale.shape[1], self.in_features // w_scale.shape[1]

@@ -1,0 +1,84 @@
+"""The native form of the quantiser and linear calls (csrc/host_calls.cpp) against the way in Python: the same bits where it takes
+the arguments, the same results and errors where it leaves them to Python."""
+import pytest
+import torch
+
+from flh_b200.nn import ActQuantizer, LinearFLH
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(monkeypatch, cuda, call):
+    """call() with the native form and without; what came out (or the error) of each."""
+    def one():
+        try:
+            out = call()
+        except (RuntimeError, IndexError, AttributeError, ValueError) as e:
+            return type(e), str(e)
+        return [t if t is None else (tuple(t.shape), t.dtype, t.stride(), t.cpu()) for t in (out if isinstance(out, tuple) else (out,))]
+    assert cuda._host is not None, "build it with python -m flh_b200.build"
+    native = one()
+    with monkeypatch.context() as m:
+        m.setattr(cuda, "_host", None)
+        plain = one()
+    return native, plain
+
+
+def _same(a, b):
+    if isinstance(a, tuple) or isinstance(b, tuple):                      # errors
+        return a == b
+    return len(a) == len(b) and all((x is None and y is None) or (x[:3] == y[:3] and torch.equal(x[3], y[3])) for x, y in zip(a, b))
+
+
+def _inputs(k, dtype):
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(6, k, device="cuda", generator=g).to(dtype)
+    yield x
+    yield x[0]                                                            # one dimension
+    yield x.view(2, 3, k)
+    yield x[:0]                                                           # no rows
+    yield x.t().contiguous().t()                                          # transposed storage
+    yield x[:, : k // 2]                                                  # row stride
+    yield x.flatten()[1:1 + 5 * k].view(5, k)                             # two bytes off
+    yield x.cpu()
+    yield x.float()
+    yield torch.nn.Parameter(x, requires_grad=False)
+
+
+@pytest.mark.parametrize("k", [64, 1024, 11008])
+@pytest.mark.parametrize("sym,group,had,dtype", [(True, 128, False, torch.float16), (True, 128, True, torch.float16), (True, 32, True, torch.bfloat16),
+                                                 (False, -1, False, torch.float16), (False, -1, True, torch.bfloat16)])
+def test_quantiser_native_equals_python(cuda, monkeypatch, k, sym, group, had, dtype):
+    quant = ActQuantizer(bits=4, group_size=group, sym=sym, use_hadamard=had, packed_output=True)
+    for x in _inputs(k, dtype):
+        native, plain = _both(monkeypatch, cuda, lambda: quant(x))
+        assert _same(native, plain), (tuple(x.shape), x.dtype, x.device, native, plain)
+
+
+@pytest.mark.parametrize("m", [1, 16, 64, 130])
+@pytest.mark.parametrize("group,zero,bias,out", [(128, False, False, None), (128, False, True, torch.bfloat16), (-1, True, True, None), (-1, False, False, torch.bfloat16)])
+def test_linear_native_equals_python(cuda, monkeypatch, m, group, zero, bias, out):
+    k, n = 1024, 512
+    g = torch.Generator(device="cuda").manual_seed(m)
+    lin = LinearFLH(k, n, bias=bias, dtype=torch.float16, device="cuda", group_size=group)
+    lin.w_packed.copy_(torch.randint(0, 256, lin.w_packed.shape, dtype=torch.uint8, device="cuda", generator=g))
+    lin.w_scale.copy_(torch.rand(lin.w_scale.shape, device="cuda", generator=g) * 0.015 + 0.005)
+    if bias:
+        lin.bias.copy_(torch.randn(n, device="cuda", generator=g))
+    x = torch.randint(0, 256, (m, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    gs = k // 128 if group == 128 else 1
+    s = (torch.rand(m, gs, device="cuda", generator=g) + 0.5).half()
+    z = torch.randint(0, 16, (m, gs), device="cuda", generator=g).half() if zero else None
+    zs = None if z is None else z.view(1, m, gs)
+    forms = [(x, s, z), (x.view(1, m, -1), s.view(1, m, gs), zs), (x[:0], s[:0], None if z is None else z[:0]),
+             (x, s.t().contiguous().t(), z)]
+    for a, b, c in forms:
+        native, plain = _both(monkeypatch, cuda, lambda: lin(a, b, c, out_dtype=out))
+        assert _same(native, plain), (tuple(a.shape), a.device, native, plain)
+    graph = torch.cuda.CUDAGraph()                                       # recorded and replayed
+    want = lin(x, s, z, out_dtype=out)
+    with torch.cuda.graph(graph):
+        y = lin(x, s, z, out_dtype=out)
+    y.zero_()
+    graph.replay()
+    assert torch.equal(y, want)
