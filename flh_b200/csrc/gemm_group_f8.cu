@@ -12,13 +12,13 @@
 // A pair of CTAs (cta_group::2) shares one 256 x BN tile, as in gemm_i8.cu: 64 KB of shared-memory traffic per CTA and
 // block instead of 96.  Per block the MMA thread fills one of two TMEM buffers while the epilogue warps fold the other.
 //
-// Measured (B200, expansion included): 2048 x 4096 -> 12288 179 us, 4096 -> 22016 292 us, 11008 -> 4096 161 us (with eight epilogue
+// Measured (B200, expansion included): 2048 x 4096 -> 12288 157 us, 4096 -> 22016 255 us, 11008 -> 4096 140 us (with eight epilogue
 // warps, one-lane issue loops and 16-byte stores in the expansion 183, 298 and 163); the converting kernel of gemm_tcgen05.cu, which
-// has the same results, 266, 439 and 247 us.  Of the 179 us 93 remain without any work in the epilogue and 110 with its TMEM loads
-// only: the epilogue is the limit.
+// has the same results, 266, 439 and 247 us.  The epilogue is the limit, and of its time what it spends on barriers counts most: a
+// wait and an arrival of each of its warps for the scales of every K-block in place of every fourth took 179 us for the first.
 //
 //   warp 0   TMA: 128 rows of A and BN / 2 rows of B per stage        warp 1   MMA issuer (the leader's)
-//   warp 2   bulk copies of a block's scales                          warps 4-19 epilogue, 32 rows x 64 columns each
+//   warp 2   bulk copies of the scales                                warps 4-19 epilogue, 32 rows x 64 columns each
 //
 // Every wait is bounded (two seconds) and reports through a status word, as in the other GEMM kernels.
 #include "tc_common.cuh"
@@ -29,7 +29,8 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 128;                  // K of a block = one group = one 128-byte swizzle row of e4m3
-constexpr int kRing = 8;                 // scale slots
+constexpr int kRing = 3;                 // scale slots
+constexpr int kSB = 4;                   // K-blocks of a scale slot: a wait and an arrival of every epilogue warp per slot
 constexpr int EW = 16;                   // epilogue warps, 32 rows x 64 columns each
 constexpr int BN = 256;                  // columns of a tile
 
@@ -127,7 +128,8 @@ struct F8Plan {
     static constexpr int kStageBytes = (BM + BN / 2) * BK;
     static constexpr int kStages = 6;
     static constexpr int kRingOff = kStages * kStageBytes;
-    static constexpr int kSlot = (BN + BM) * 4;           // weight scales, then token scales
+    static constexpr int kScales = (BN + BM) * 4;         // of a K-block: weight scales, then token scales
+    static constexpr int kSlot = kSB * kScales;
     static constexpr int kBarOff = kRingOff + kRing * kSlot;
     static constexpr int kBytes = kBarOff + 512 + 1024;   // barriers, then slack to align the base to 1024
     static constexpr int kThreads = 128 + 32 * EW;
@@ -218,15 +220,19 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             bool ok = true;
             for (int tile = first; tile < p.num_tiles; tile += step) {
                 const float *sa = p.sa + (tile % p.m_blocks) * 2 * BM + (int)rank * BM, *sb = p.sb + (tile / p.m_blocks) * BN;
-                for (int kb = 0; kb < KB; ++kb, sa += p.Mp, sb += p.N) {
+                for (int kb = 0; kb < KB; kb += kSB) {
+                    const int nb = min(kSB, KB - kb);
                     ok = __all_sync(0xffffffffu, ok && wait_f8(sempty(slot), ph, abort_flag, 44));
                     const uint32_t dst = base + Plan::kRingOff + slot * Plan::kSlot;
                     if (ok && elect_one()) {
-                        mbar_expect_tx(sfull(slot), Plan::kSlot);
-                        bulk_load(dst, sb, BN * 4, sfull(slot));
-                        bulk_load(dst + BN * 4, sa, BM * 4, sfull(slot));
+                        mbar_expect_tx(sfull(slot), nb * Plan::kScales);
+                        for (int b = 0; b < nb; ++b) {
+                            bulk_load(dst + b * Plan::kScales, sb + (long)b * p.N, BN * 4, sfull(slot));
+                            bulk_load(dst + b * Plan::kScales + BN * 4, sa + (long)b * p.Mp, BM * 4, sfull(slot));
+                        }
                     }
                     __syncwarp();
+                    sa += (long)kSB * p.Mp; sb += (long)kSB * p.N;
                     it += ok;
                     if (++slot == kRing) { slot = 0; ph ^= 1; }
                 }
@@ -270,7 +276,8 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const int wq = warp & 3;                         // TMEM lane quarter this warp may read
         const int c0 = ((warp - 4) >> 2) * COLS;         // first tile column of this warp
         const uint32_t tlane = tmem + ((uint32_t)(wq * 32) << 16) + c0;
-        int it = 0;
+        int it = 0, slot = 0;
+        uint32_t sph = 0;
         bool ok = true;
         // The outcome of every wait is made warp-uniform by a vote, and a warp that gave up keeps walking the loops (no
         // waits, no TMEM reads, no stores): warp-wide tcgen05.ld never runs in a diverged warp.
@@ -285,8 +292,8 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 for (int n = 0; n < COLS / 8; ++n) acc[r][n] = 0ull;
 #pragma unroll 1
             for (int kb = 0; kb < KB; ++kb, ++it) {
-                const int buf = it & 1, slot = it % kRing;
-                ok = __all_sync(0xffffffffu, ok && wait_f8(sfull(slot), (it / kRing) & 1, abort_flag, 45) &&
+                const int buf = it & 1, sub = kb % kSB;
+                ok = __all_sync(0xffffffffu, ok && (sub != 0 || wait_f8(sfull(slot), sph, abort_flag, 45)) &&
                                                  wait_f8(acc_full(buf), (it >> 1) & 1, abort_flag, 46));
                 auto release_acc = [&]() {               // the accumulator is in registers: the tensor core may have the buffer
                     tc_fence_before();
@@ -294,7 +301,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     if (lane == 0) { if (rank == 1) mbar_arrive_remote(acc_empty(buf), 0); else mbar_arrive(acc_empty(buf)); }
                 };
                 if (ok) {
-                    const float *sl = reinterpret_cast<const float *>(sm + Plan::kRingOff + slot * Plan::kSlot);
+                    const float *sl = reinterpret_cast<const float *>(sm + Plan::kRingOff + slot * Plan::kSlot + sub * Plan::kScales);
                     const uint32_t src = tlane + buf * 256;
                     tc_fence_after();
                     // the next 16 columns are on their way from TMEM while these are folded
@@ -325,8 +332,11 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 } else {
                     release_acc();
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(sempty(slot));
+                if (sub == kSB - 1 || kb == KB - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sempty(slot));
+                    if (++slot == kRing) { slot = 0; sph ^= 1; }
+                }
             }
             // Four lanes hold a row's columns two by two: they exchange 4 x 4 words so that each has eight neighbours (one 16-byte
             // store; four lanes then write 64 bytes of a row).
