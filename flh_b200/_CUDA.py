@@ -264,6 +264,12 @@ def act_quant_token(x, hadamard: bool, clip: float):
     return q, s, z
 
 
+def square_f32(x):
+    """x * x in binary32, the bits of x.float().pow(2), in one pass: x a contiguous CUDA float16 or bfloat16 tensor whose numel is a
+    multiple of 8 and of which no derivative is taken; None for anything else."""
+    return None if _host is None else _host.square(x)
+
+
 def silu_mul(gu):
     """SiLU(gate) * up of the merged gate/up GEMM output gu [M, 2F] (row stride allowed) -> [M, F] (include/flh_b200.h)."""
     _check(gu.is_cuda and gu.dtype in (torch.float16, torch.bfloat16), "gu must be a CUDA float16 or bfloat16 tensor")

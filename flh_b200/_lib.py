@@ -23,6 +23,7 @@ SIGNATURES = {
     "flh_b200_quant_token_asym_i4": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_int, c_int, c_void_p, c_float,
                                              c_void_p, c_void_p, c_void_p, c_void_p]),
     "flh_b200_quant_token_kernel": (ctypes.c_char_p, [c_long, c_long, c_int, c_int]),
+    "flh_b200_square_f32": (c_int, [c_void_p, c_int, c_long, c_void_p, c_void_p]),
     "flh_b200_silu_mul": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_void_p, c_void_p]),
     "flh_b200_silu_mul_quant_token_asym_i4": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_int, c_int, c_void_p, c_float,
                                                       c_void_p, c_void_p, c_void_p, c_void_p]),

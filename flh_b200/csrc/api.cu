@@ -61,6 +61,7 @@ int quant_token_factor_status(int *);
 int quant_token_factor_status_clear();
 const char *quant_token_kernel_name(long, long, int, int);
 int launch_silu_mul(const void *, int, long, long, long, void *, cudaStream_t);
+int launch_square(const void *, int, long, void *, cudaStream_t);
 int launch_silu_mul_quant_token_tc(const void *, int, long, long, long, int, const uint32_t *, float, uint8_t *, void *, void *, cudaStream_t);
 int launch_rope_kv(const void *, const float *, const float *, void *, void *, void *, int, int, int, int, int, int, int, int, cudaStream_t);
 int quant_token_tc_status(int *);
@@ -214,6 +215,15 @@ int flh_b200_silu_mul(const void *gu, int in_dtype, long M, long F, long ld, voi
     FLH_REQUIRE(gu && out, FLH_B200_EINVAL, "null pointer");
     FLH_REQUIRE(aligned16(gu) && aligned16(out), FLH_B200_EALIGN, "gu and out must be 16-byte aligned");
     return launch_silu_mul(gu, in_dtype, M, F, ld, out, static_cast<cudaStream_t>(stream));
+}
+
+int flh_b200_square_f32(const void *x, int in_dtype, long n, void *out, void *stream) {
+    FLH_REQUIRE(n >= 0 && n % 8 == 0, FLH_B200_EINVAL, "n must be a multiple of 8 (got %ld)", n);
+    FLH_REQUIRE(in_dtype == FLH_B200_F16 || in_dtype == FLH_B200_BF16, FLH_B200_EINVAL, "in_dtype must be F16 or BF16");
+    if (n == 0) return 0;
+    FLH_REQUIRE(x && out, FLH_B200_EINVAL, "null pointer");
+    FLH_REQUIRE(aligned16(x) && (reinterpret_cast<uintptr_t>(out) & 31) == 0, FLH_B200_EALIGN, "x must be 16-byte, out 32-byte aligned");
+    return launch_square(x, in_dtype, n, out, static_cast<cudaStream_t>(stream));
 }
 
 int flh_b200_silu_mul_quant_token_asym_i4(const void *gu, int in_dtype, long M, long F, long ld, int hadamard, int kfac,

@@ -9,6 +9,7 @@
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -141,7 +142,24 @@ PyObject *gemm(PyObject *, PyObject *const *args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// square(x) -> x * x in binary32, for values that no derivative is taken of
+PyObject *square(PyObject *, PyObject *x_) {
+    HANDLE_TH_ERRORS
+    const at::Tensor *x = tensor(x_);
+    if (!x || observed() || (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16)) Py_RETURN_NONE;
+    const c10::DeviceIndex dev = c10::cuda::current_device();
+    if (!plain(*x, dev) || x->numel() % 8 || reinterpret_cast<uintptr_t>(x->data_ptr()) % 16) Py_RETURN_NONE;
+    if ((c10::GradMode::is_enabled() && x->requires_grad()) || x->_fw_grad(0).defined()) Py_RETURN_NONE;
+    at::Tensor y = empty(x->sizes(), at::kFloat, *x);
+    const int rc = flh_b200_square_f32(x->data_ptr(), x->scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, x->numel(), y.data_ptr(),
+                                       c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc) return failed("square_f32", rc);
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"square", square, METH_O, nullptr},
     {"act_quant_group", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(act_quant_group)), METH_FASTCALL, nullptr},
     {"act_quant_token", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(act_quant_token)), METH_FASTCALL, nullptr},
     {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(gemm)), METH_FASTCALL, nullptr},

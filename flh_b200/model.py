@@ -79,8 +79,13 @@ class RMSNorm(torch.nn.Module):
     def forward(self, x, last=False):
         """last: only the last position of x [B, S, K].  The mean is over all positions even then: the order in which a
         reduction sums a row depends on the number of rows, and the result has the bits of the whole norm's last position."""
-        v = x.float()
-        c = torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
+        squares = _CUDA.square_f32(x) if last else None
+        if squares is None:
+            v = x.float()
+            squares = v.pow(2)
+        else:
+            v = x[:, -1:].float()
+        c = torch.rsqrt(squares.mean(-1, keepdim=True) + self.eps)
         if last:
             v, c = v[:, -1:], c[:, -1:]
         return (v * c).to(x.dtype) * self.weight

@@ -144,6 +144,10 @@ int flh_b200_rmsnorm_quant_group_sym_i4(const void *x, long M, long K, float eps
  * The reference runs act_fn and the product as separate PyTorch kernels (modeling_llama.py:524). */
 int flh_b200_silu_mul(const void *gu, int in_dtype, long M, long F, long ld, void *out, void *stream);
 
+/* out[i] = (float)x[i] * (float)x[i] for n contiguous f16 or bf16 values, out binary32: the squares of an RMS-norm in one pass
+ * instead of a widened copy and its square.  n % 8 == 0, x 16-byte aligned, out 32-byte aligned. */
+int flh_b200_square_f32(const void *x, int in_dtype, long n, void *out, void *stream);
+
 /* The same followed by the full-width transform and the per-token asymmetric quantiser of flh_b200_quant_token_asym_i4
  * (hadamard = 1), as ONE kernel: the MLP's "act_fn(gate) * up -> quantizer2" (modeling_llama.py:524-525) with the online
  * transform of the per-token mode.  The product never reaches global memory: the epilogue warps of the tensor-core

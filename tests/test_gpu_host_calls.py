@@ -24,6 +24,21 @@ def _both(monkeypatch, cuda, call):
     return native, plain
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 8), (2, 3, 4096), (5, 257, 1032)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_squares_and_final_norm(cuda, monkeypatch, shape, dtype):
+    from flh_b200.model import RMSNorm
+    x = (torch.randn(shape, device="cuda") * 8).to(dtype)
+    x.view(-1)[:4] = torch.tensor([0.0, -0.0, float("inf"), 6e-8], dtype=dtype)
+    assert torch.equal(cuda.square_f32(x), x.float().pow(2))
+    norm = RMSNorm(shape[-1], 1e-5).cuda()
+    x = x.nan_to_num(posinf=1.0)
+    assert torch.equal(norm(x, last=True), norm(x)[:, -1:])
+    grad = x.clone().requires_grad_()                    # a derivative has to pass through
+    assert cuda.square_f32(grad) is None and norm(grad, last=True).requires_grad
+    assert cuda.square_f32(x[..., 1:]) is None and cuda.square_f32(x.float()) is None and cuda.square_f32(x.cpu()) is None
+
+
 def _same(a, b):
     if isinstance(a, tuple) or isinstance(b, tuple):                      # errors
         return a == b
