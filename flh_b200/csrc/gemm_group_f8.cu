@@ -12,10 +12,11 @@
 // A pair of CTAs (cta_group::2) shares one 256 x BN tile, as in gemm_i8.cu: 64 KB of shared-memory traffic per CTA and
 // block instead of 96.  Per block the MMA thread fills one of two TMEM buffers while the epilogue warps fold the other.
 //
-// Measured (B200, expansion included): 2048 x 4096 -> 12288 157 us, 4096 -> 22016 255 us, 11008 -> 4096 140 us (with eight epilogue
-// warps, one-lane issue loops and 16-byte stores in the expansion 183, 298 and 163); the converting kernel of gemm_tcgen05.cu, which
-// has the same results, 266, 439 and 247 us.  The epilogue is the limit, and of its time what it spends on barriers counts most: a
-// wait and an arrival of each of its warps for the scales of every K-block in place of every fourth took 179 us for the first.
+// Measured (B200, expansion included): 2048 x 4096 -> 12288 146 us, 4096 -> 22016 235 us, 11008 -> 4096 130 us; the converting kernel
+// of gemm_tcgen05.cu, which has the same results, 266, 439 and 247 us.  The epilogue is the limit, and of its time what it spends on
+// barriers counts most.  For the first shape: eight epilogue warps and issue loops walked by one lane 183; sixteen warps 179; their
+// wait and arrival for the scales of every fourth K-block in place of each 157; waits with one outcome for the warp (mbar_wait_warp)
+// and the leader's barrier mapped once 146.
 //
 //   warp 0   TMA: 128 rows of A and BN / 2 rows of B per stage        warp 1   MMA issuer (the leader's)
 //   warp 2   bulk copies of the scales                                warps 4-19 epilogue, 32 rows x 64 columns each
@@ -37,7 +38,7 @@ constexpr int BN = 256;                  // columns of a tile
 __device__ int g_status_f8[4];
 
 __device__ __forceinline__ bool wait_f8(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code) {
-    return mbar_wait_status(g_status_f8, bar, parity, abort_flag, code);
+    return mbar_wait_warp(g_status_f8, bar, parity, abort_flag, code);
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -189,7 +190,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 const int m0 = (tile % p.m_blocks) * 2 * BM + (int)rank * BM;
                 const int n0 = (tile / p.m_blocks) * BN + (int)rank * (BN / 2);
                 for (int kb = 0; kb < KB; ++kb) {
-                    ok = __all_sync(0xffffffffu, ok && wait_f8(empty(s), ph, abort_flag, 41));
+                    ok = ok && wait_f8(empty(s), ph, abort_flag, 41);
                     const uint32_t dst = base + s * Plan::kStageBytes;
                     if (ok && elect_one()) {
                         if (rank == 1) {
@@ -222,7 +223,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 const float *sa = p.sa + (tile % p.m_blocks) * 2 * BM + (int)rank * BM, *sb = p.sb + (tile / p.m_blocks) * BN;
                 for (int kb = 0; kb < KB; kb += kSB) {
                     const int nb = min(kSB, KB - kb);
-                    ok = __all_sync(0xffffffffu, ok && wait_f8(sempty(slot), ph, abort_flag, 44));
+                    ok = ok && wait_f8(sempty(slot), ph, abort_flag, 44);
                     const uint32_t dst = base + Plan::kRingOff + slot * Plan::kSlot;
                     if (ok && elect_one()) {
                         mbar_expect_tx(sfull(slot), nb * Plan::kScales);
@@ -253,8 +254,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             for (int tile = first; tile < p.num_tiles; tile += step) {
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int buf = it & 1;
-                    ok = __all_sync(0xffffffffu, ok && wait_f8(full(s), ph, abort_flag, 43) &&
-                                                     wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42));
+                    ok = ok && wait_f8(full(s), ph, abort_flag, 43) && wait_f8(acc_empty(buf), ((it >> 1) & 1) ^ 1, abort_flag, 42);
                     tc_fence_after();
                     const uint32_t a_addr = base + s * Plan::kStageBytes;
                     const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BM * BK);
@@ -276,6 +276,7 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const int wq = warp & 3;                         // TMEM lane quarter this warp may read
         const int c0 = ((warp - 4) >> 2) * COLS;         // first tile column of this warp
         const uint32_t tlane = tmem + ((uint32_t)(wq * 32) << 16) + c0;
+        const uint32_t leader_empty = map_to_leader(acc_empty(0));
         int it = 0, slot = 0;
         uint32_t sph = 0;
         bool ok = true;
@@ -293,12 +294,11 @@ gemm_group_f8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll 1
             for (int kb = 0; kb < KB; ++kb, ++it) {
                 const int buf = it & 1, sub = kb % kSB;
-                ok = __all_sync(0xffffffffu, ok && (sub != 0 || wait_f8(sfull(slot), sph, abort_flag, 45)) &&
-                                                 wait_f8(acc_full(buf), (it >> 1) & 1, abort_flag, 46));
+                ok = ok && (sub != 0 || wait_f8(sfull(slot), sph, abort_flag, 45)) && wait_f8(acc_full(buf), (it >> 1) & 1, abort_flag, 46);
                 auto release_acc = [&]() {               // the accumulator is in registers: the tensor core may have the buffer
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) { if (rank == 1) mbar_arrive_remote(acc_empty(buf), 0); else mbar_arrive(acc_empty(buf)); }
+                    if (lane == 0) mbar_arrive_cluster(leader_empty + 8u * buf);
                 };
                 if (ok) {
                     const float *sl = reinterpret_cast<const float *>(sm + Plan::kRingOff + slot * Plan::kSlot + sub * Plan::kScales);

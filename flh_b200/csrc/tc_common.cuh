@@ -61,6 +61,12 @@ __device__ __forceinline__ bool mbar_wait_status(int *status, uint32_t bar, uint
         }
     }
 }
+// The same for a converged warp, with one outcome for all its lanes.  A try that succeeds at once, as most do, costs a vote and a
+// uniform branch; the loop behind it is not woven into the warp's control flow.
+__device__ __forceinline__ bool mbar_wait_warp(int *status, uint32_t bar, uint32_t parity, volatile int *abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait_status(status, bar, parity, abort_flag, code));
+}
 // One lane of a converged warp.  A loop that issues tcgen05 or TMA instructions is walked by its whole warp, and only the instructions
 // themselves are under this predicate: their operands are uniform registers, and in a loop that one lane walks (if (lane == 0)) each is
 // moved there again with the warp's divergence to manage.  Measured for an iteration of two waits, four MMAs and two commits: 596 clocks
@@ -97,15 +103,9 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
                    "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                  : "r"(taddr) : "memory");
 }
-// 16 lanes x 32 columns in the layout of an mma.sync accumulator: v[4 n + 0 / 1] = lane i / 4, columns 8 n + 2 (i % 4) and the next,
-// v[4 n + 2 / 3] the same columns of lane i / 4 + 8
-__device__ __forceinline__ void tc_ld_frag(uint32_t taddr, uint32_t *v) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr) : "memory");
-}
-// the same, 16 lanes x 16 columns
+// 16 lanes x 16 columns in the layout of an mma.sync accumulator: v[4 n + 0 / 1] = lane i / 4, columns 8 n + 2 (i % 4) and the next,
+// v[4 n + 2 / 3] the same columns of lane i / 4 + 8.  (32 columns per instruction, .x4, come at half the rate: 522 against 276 clocks for
+// 128 x 256 values.)
 __device__ __forceinline__ void tc_ld_frag2(uint32_t taddr, uint32_t *v) {
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");

@@ -23,6 +23,15 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) 
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(bar), "r"(rank));
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(raddr) : "memory");
 }
+// the same in two parts, for a barrier that is arrived at again and again: its address in CTA 0, then the arrival
+__device__ __forceinline__ uint32_t map_to_leader(uint32_t bar) {
+    uint32_t raddr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(raddr) : "r"(bar));
+    return raddr;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t raddr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(raddr) : "memory");
+}
 // TMA tile load of a CTA of a pair whose completion is counted on the barrier at the same offset in CTA 0
 __device__ __forceinline__ void tma_load_2d_to_leader(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
     uint32_t rbar;
