@@ -302,16 +302,17 @@ static int pick_stream(long M, long N, long K) {
 
 // Batches with group-128 scales for which expanding both operands first pays for itself.  Both kernels walk whole waves of tiles
 // and both are bound by a time per 128-K block (measured on B200: 1.42 us for a wave of 148 tiles of 128 x 256 in the converting
-// kernel, 0.9 us for a wave of 74 pairs on 256 x 256 here); the expansion moves 1.5 bytes per code of either operand at 4.3 TB/s
-// and its launch costs 2 us.  The estimate and the measurements agree on who wins (us, converting / expanded): 384 rows
-// 4096 -> 12288 48 / 76, 512 rows 91 / 76, 65 rows 11008 -> 4096 122 / 86, 384 rows 8192 -> 57344 483 / 500, 512 rows 669 / 501,
-// 512 rows 1024 -> 8192 15 / 17, 1024 rows 27 / 25; narrow outputs, where the rows are what is expanded: 8192 -> 256 with 8,192
-// rows 98 / 79, with 16,384 rows 100 / 104; 4096 -> 256 with 16,384 rows 47 / 55, 8192 -> 512 196 / 155.
+// kernel, 0.63 us for a wave of 74 pairs on 256 x 256 here); the expansion moves 1.5 bytes per code of either operand at 4.3 TB/s, and
+// the two launches cost 5 us more than one.  The estimate and the measurements agree on who wins, but for two shapes 2 % apart, in
+// the 102 of 65 to 8,192 rows, K = 1024 to 28672 and N = 256 to 57344 that were timed (us, converting / expanded): 256 rows 4096 -> 12288 46 / 37, 384
+// rows 47 / 58, 512 rows 90 / 58; 65 rows 11008 -> 4096 123 / 69; 65 rows 8192 -> 57344 182 / 279, 384 rows 483 / 399; 384 rows
+// 4096 -> 22016 90 / 88 (converting); 512 rows 1024 -> 8192 15 / 17; narrow outputs, where the rows are what is expanded: 8192 -> 256 with 8,192
+// rows 98 / 60, 4096 -> 512 46 / 33.
 static bool group_f8_pays(long M, long N, long K, long a_group, long b_group) {
     if ((a_group < b_group ? a_group : b_group) != 128 || K <= 128 || M <= 64 || !gemm_group_f8_supported(M, N, K)) return false;
     const long kb = K / 128, pairs = kNumSMs / 2;
     const long waves = ((M + 255) / 256 * (N / 256) + pairs - 1) / pairs, waves_tc = ((M + 127) / 128 * (N / 256) + kNumSMs - 1) / kNumSMs;
-    return 0.9 * waves * kb + 0.35e-6 * (M + N) * K + 2.0 < 1.42 * waves_tc * kb;
+    return 0.63 * waves * kb + 0.35e-6 * (M + N) * K + 5.0 < 1.42 * waves_tc * kb;
 }
 
 int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) {
