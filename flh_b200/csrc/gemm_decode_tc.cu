@@ -41,10 +41,11 @@ __device__ unsigned long long g_wait_ns[8];
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code,
                                           unsigned long long *waited = nullptr) {
-    // a try may already sleep in hardware, so what does not succeed at once is timed as a whole
-    if (mbar_test(bar, parity)) return true;
+    // by whole warps, with one outcome for all lanes; a try may already sleep in hardware, so what does not succeed at once is timed
+    // as a whole
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
     const uint64_t t0 = waited ? gtimer() : 0;
-    const bool ok = mbar_wait_status(g_status, bar, parity, abort_flag, code);
+    const bool ok = __all_sync(0xffffffffu, mbar_wait_status(g_status, bar, parity, abort_flag, code));
     if (waited) *waited += gtimer() - t0;
     return ok;
 }
@@ -60,17 +61,22 @@ struct DecParams {
     float *partials;                    // [2 * grid][TOK][128]
 };
 
-template <int TOK, bool GROUPED>
+// KP: K-blocks of a step.  Every stage and every accumulator that changes hands costs its warps a wait and an arrival; with group
+// scales and 64 tokens, where one CTA has the SM, two K-blocks change hands at a time (K and the CTAs' ranges being
+// multiples of two; not with zero-points, whose terms leave no registers for it).
+// 64 tokens, 8192 -> 28672, group scales, quantiser included: 68.7 -> 63.2 us; more epilogue or converter warps, which do more barrier
+// operations: 79.
+template <int TOK, bool GROUPED, int KP>
 struct DecPlan {
     static constexpr bool kTwo = TOK <= 32;                 // two CTAs per SM
-    static constexpr int SP = TOK == 16 ? 7 : (TOK == 32 ? 6 : 10);  // packed stages in flight (TMA)
-    static constexpr int SE = kTwo ? 2 : 3;                 // expanded stages
+    static constexpr int SP = TOK == 16 ? 7 : (TOK == 32 ? 6 : (KP == 2 ? 4 : 10));  // packed stages in flight (TMA)
+    static constexpr int SE = kTwo || KP == 2 ? 2 : 3;      // expanded stages
     static constexpr int NBUF = GROUPED ? 4 : 2;            // TMEM accumulators
     static constexpr int EG = TOK == 64 ? 2 : 1;            // epilogue groups of four warps, TOK / EG token columns each
     static constexpr int kThreads = 192 + 128 * EG;
-    static constexpr int kTmemCols = NBUF * TOK < 32 ? 32 : NBUF * TOK;
-    static constexpr int kPkStage = (BR + TOK) * (BK / 2);
-    static constexpr int kExStage = (BR + TOK) * BK;
+    static constexpr int kTmemCols = NBUF * KP * TOK < 32 ? 32 : NBUF * KP * TOK;
+    static constexpr int kPkBlock = (BR + TOK) * (BK / 2), kPkStage = KP * kPkBlock;
+    static constexpr int kExBlock = (BR + TOK) * BK, kExStage = KP * kExBlock;
     static constexpr int kExOff = 0;
     static constexpr int kPkOff = SE * kExStage;
     static constexpr int kBarOff = kPkOff + SP * kPkStage;
@@ -91,11 +97,11 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&v)[TOK])
     }
 }
 
-template <int TOK, bool GROUPED, bool A_UNSIGNED>
-__global__ void __launch_bounds__((DecPlan<TOK, GROUPED>::kThreads), TOK <= 32 ? 2 : 1)
+template <int TOK, bool GROUPED, bool A_UNSIGNED, int KP>
+__global__ void __launch_bounds__((DecPlan<TOK, GROUPED, KP>::kThreads), TOK <= 32 ? 2 : 1)
 gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                       const DecParams p) {
-    using Plan = DecPlan<TOK, GROUPED>;
+    using Plan = DecPlan<TOK, GROUPED, KP>;
     constexpr int SP = Plan::SP, SE = Plan::SE, NBUF = Plan::NBUF, EG = Plan::EG, TE = TOK / EG;
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t raw = smem_u32(smem_dyn);
@@ -118,7 +124,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int KB = p.KB;
     const int lin_begin = blockIdx.x * p.per;
     const int lin_end = min(p.total, lin_begin + p.per);
-    const int count = lin_end - lin_begin;          // K-blocks this CTA streams (> 0 by the choice of the grid)
+    const int count = lin_end - lin_begin;          // K-blocks this CTA streams (> 0 by the choice of the grid; a multiple of KP)
+    const int steps = count / KP;
 
     // token scales (and zero-points) of the whole K: [group][token] with group scales on the token side, [token]
     // otherwise; tokens past M read as zero.  The epilogue warps stage them while the first tiles are in flight.
@@ -151,16 +158,19 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         int it = 0, s = 0;
         uint32_t ph = 1;
         unsigned long long w1 = 0;
-        for (; it < count; ++it) {
-            if (!__all_sync(0xffffffffu, mbar_wait(pk_empty(s), ph, abort_flag, 1, &w1))) break;
+        for (; it < steps; ++it) {
+            if (!mbar_wait(pk_empty(s), ph, abort_flag, 1, &w1)) break;
             const uint32_t dst = base + Plan::kPkOff + s * Plan::kPkStage;
             if (elect_one()) {
                 mbar_expect_tx(pk_full(s), Plan::kPkStage);
-                tma_load_2d(dst, &map_w, kb * (BK / 2), tile * BR, pk_full(s));
-                tma_load_2d(dst + BR * (BK / 2), &map_x, kb * (BK / 2), 0, pk_full(s));
+#pragma unroll
+                for (int q = 0; q < KP; ++q) {
+                    tma_load_2d(dst + q * Plan::kPkBlock, &map_w, (kb + q) * (BK / 2), tile * BR, pk_full(s));
+                    tma_load_2d(dst + q * Plan::kPkBlock + BR * (BK / 2), &map_x, (kb + q) * (BK / 2), 0, pk_full(s));
+                }
             }
             __syncwarp();
-            if (++kb == KB) { kb = 0; ++tile; }
+            if ((kb += KP) == KB) { kb = 0; ++tile; }
             if (++s == SP) { s = 0; ph ^= 1; }
         }
         if (lane == 0) atomicAdd(&g_wait_ns[1], w1);
@@ -180,28 +190,31 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         int u = 0, s = 0;
         uint32_t ph = 0;
         unsigned long long w2 = 0, w3 = 0;
-        for (int it = 0; it < count; ++it) {
+        for (int it = 0; it < steps; ++it) {
             const int buf = u % NBUF;
             const bool seg_first = it == 0 || kb == 0;
-            const bool seg_last = it == count - 1 || kb == KB - 1;
+            const bool seg_last = it == steps - 1 || kb == KB - KP;
             bool ok = true;
             if ((GROUPED || seg_first) && u >= NBUF) ok = mbar_wait(acc_empty(buf), ((u / NBUF) & 1) ^ 1, abort_flag, 2, &w2);
-            if (!__all_sync(0xffffffffu, ok && mbar_wait(ex_full(s), ph, abort_flag, 3, &w3))) break;
+            if (!ok || !mbar_wait(ex_full(s), ph, abort_flag, 3, &w3)) break;
             tc_fence_after();
-            const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage;
-            const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
             if (elect_one()) {
 #pragma unroll
-                for (int k4 = 0; k4 < BK / 32; ++k4) {
-                    const uint32_t accum = GROUPED ? (k4 > 0) : (!seg_first || k4 > 0);
-                    tc_mma_i8(tmem + buf * TOK, adesc + 2 * k4, bdesc + 2 * k4, idesc, accum);
+                for (int q = 0; q < KP; ++q) {
+                    const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage + q * Plan::kExBlock;
+                    const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
+#pragma unroll
+                    for (int k4 = 0; k4 < BK / 32; ++k4) {
+                        const uint32_t accum = GROUPED ? (k4 > 0) : (!seg_first || k4 > 0);
+                        tc_mma_i8(tmem + (buf * KP + q) * TOK, adesc + 2 * k4, bdesc + 2 * k4, idesc, accum);
+                    }
                 }
                 tc_commit(ex_empty(s));
                 if (GROUPED || seg_last) tc_commit(acc_full(buf));
             }
             __syncwarp();
             if (GROUPED || seg_last) ++u;
-            if (++kb == KB) kb = 0;
+            if ((kb += KP) == KB) kb = 0;
             if (++s == SE) { s = 0; ph ^= 1; }
         }
         if (lane == 0) { atomicAdd(&g_wait_ns[2], w2); atomicAdd(&g_wait_ns[3], w3); }
@@ -219,26 +232,29 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             ex_off[j] = row * 128 + (((2 * c) ^ (row & 7)) << 4);
         }
         unsigned long long w4 = 0, w5 = 0;
-        for (int it = 0; it < count; ++it) {
+        for (int it = 0; it < steps; ++it) {
             const int sp = it % SP, se = it % SE;
-            if (!__all_sync(0xffffffffu, mbar_wait(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4) &&
-                                             mbar_wait(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5))) break;
+            if (!mbar_wait(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4)) break;
+            if (!mbar_wait(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5)) break;
             const uint8_t *pk = sm + Plan::kPkOff + sp * Plan::kPkStage;
             uint8_t *ex = sm + Plan::kExOff + se * Plan::kExStage;
-            uint4 wv[kPerT];
 #pragma unroll
-            for (int j = 0; j < kPerT; ++j)
-                if (pk_off[j] >= 0) wv[j] = *reinterpret_cast<const uint4 *>(pk + pk_off[j]);
+            for (int q = 0; q < KP; ++q, pk += Plan::kPkBlock, ex += Plan::kExBlock) {
+                uint4 wv[kPerT];
 #pragma unroll
-            for (int j = 0; j < kPerT; ++j) {
-                if (pk_off[j] >= 0) {
-                    const uint4 w = wv[j];
-                    uint4 e, o;
-                    e.x = (w.x << 4) & 0xF0F0F0F0u; e.y = (w.y << 4) & 0xF0F0F0F0u;
-                    e.z = (w.z << 4) & 0xF0F0F0F0u; e.w = (w.w << 4) & 0xF0F0F0F0u;
-                    o.x = w.x & 0xF0F0F0F0u; o.y = w.y & 0xF0F0F0F0u; o.z = w.z & 0xF0F0F0F0u; o.w = w.w & 0xF0F0F0F0u;
-                    *reinterpret_cast<uint4 *>(ex + ex_off[j]) = e;            // 16-byte chunk 2c   ^ (row & 7)
-                    *reinterpret_cast<uint4 *>(ex + (ex_off[j] ^ 16)) = o;     // 16-byte chunk 2c+1 ^ (row & 7)
+                for (int j = 0; j < kPerT; ++j)
+                    if (pk_off[j] >= 0) wv[j] = *reinterpret_cast<const uint4 *>(pk + pk_off[j]);
+#pragma unroll
+                for (int j = 0; j < kPerT; ++j) {
+                    if (pk_off[j] >= 0) {
+                        const uint4 w = wv[j];
+                        uint4 e, o;
+                        e.x = (w.x << 4) & 0xF0F0F0F0u; e.y = (w.y << 4) & 0xF0F0F0F0u;
+                        e.z = (w.z << 4) & 0xF0F0F0F0u; e.w = (w.w << 4) & 0xF0F0F0F0u;
+                        o.x = w.x & 0xF0F0F0F0u; o.y = w.y & 0xF0F0F0F0u; o.z = w.z & 0xF0F0F0F0u; o.w = w.w & 0xF0F0F0F0u;
+                        *reinterpret_cast<uint4 *>(ex + ex_off[j]) = e;            // 16-byte chunk 2c   ^ (row & 7)
+                        *reinterpret_cast<uint4 *>(ex + (ex_off[j] ^ 16)) = o;     // 16-byte chunk 2c+1 ^ (row & 7)
+                    }
                 }
             }
             fence_proxy_async();
@@ -292,41 +308,58 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (GROUPED) {
                 // 256 * sum arrives from the tensor core; without zero-points the 1/256 rides in the weight scale
                 const float unit = A_UNSIGNED ? 1.0f : (1.0f / 256.0f);
-                float sbv = __half2float(p.b_scale[(long)n * p.gb_cols + gbs * kb0]) * unit;
-                int rsv = A_UNSIGNED ? p.b_rowsum[(long)n * KB + kb0] : 0;
-                for (int kb = kb0; kb < kb1; ++kb, ++u) {
-                    float nsb = sbv;
-                    int nrs = rsv;
-                    if (kb + 1 < kb1) {                  // the next group's channel data, fetched early
-                        if (gbs) nsb = __half2float(p.b_scale[(long)n * p.gb_cols + kb + 1]) * unit;
-                        if (A_UNSIGNED) nrs = p.b_rowsum[(long)n * KB + kb + 1];
-                    }
-                    const int buf = u % NBUF;
-                    ok = __all_sync(0xffffffffu, ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 6, &w6));
-                    tc_fence_after();
-                    uint32_t v[TE];
-                    if (ok) { tmem_ld_cols<TE>(tlane + buf * TOK + j0, v); tc_wait_ld(); }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty(buf));
-                    if (ok) {
-                        const float *sa = sa_s + gas * kb + j0;
-                        const int *za = za_s + gas * kb + j0;
-                        const uint64_t sb2 = pack2(sbv, sbv);
+                const __half *bs = p.b_scale + (long)n * p.gb_cols;
+                const int32_t *br = A_UNSIGNED ? p.b_rowsum + (long)n * KB : nullptr;
+                float sbv[KP];
+                int rsv[KP];
 #pragma unroll
-                        for (int j = 0; j < TE; j += 2) {
-                            const float2 sap = *reinterpret_cast<const float2 *>(sa + j);
-                            int i0 = (int)v[j], i1 = (int)v[j + 1];
-                            if (A_UNSIGNED) { i0 = (i0 >> 8) - za[j] * rsv; i1 = (i1 >> 8) - za[j + 1] * rsv; }
-                            const uint64_t p2 = mul2(pack2(sap.x, sap.y), sb2);
-                            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(accf[j >> 1]) : "l"(pack2((float)i0, (float)i1)), "l"(p2));
+                for (int q = 0; q < KP; ++q) {
+                    sbv[q] = __half2float(bs[gbs * (kb0 + q)]) * unit;
+                    rsv[q] = A_UNSIGNED ? br[kb0 + q] : 0;
+                }
+                for (int kb = kb0; kb < kb1; kb += KP, ++u) {
+                    float nsb[KP];
+                    int nrs[KP];
+#pragma unroll
+                    for (int q = 0; q < KP; ++q) {       // the next step's channel data, fetched early
+                        nsb[q] = sbv[q]; nrs[q] = rsv[q];
+                        if (kb + KP < kb1) {
+                            if (gbs) nsb[q] = __half2float(bs[kb + KP + q]) * unit;
+                            if (A_UNSIGNED) nrs[q] = br[kb + KP + q];
                         }
                     }
-                    sbv = nsb; rsv = nrs;
+                    const int buf = u % NBUF;
+                    ok = ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 6, &w6);
+                    tc_fence_after();
+#pragma unroll
+                    for (int q = 0; q < KP; ++q) {
+                        uint32_t v[TE];
+                        if (ok) { tmem_ld_cols<TE>(tlane + (buf * KP + q) * TOK + j0, v); tc_wait_ld(); }
+                        if (q == KP - 1) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(acc_empty(buf));
+                        }
+                        if (ok) {
+                            const float *sa = sa_s + gas * (kb + q) + j0;
+                            const int *za = za_s + gas * (kb + q) + j0;
+                            const uint64_t sb2 = pack2(sbv[q], sbv[q]);
+#pragma unroll
+                            for (int j = 0; j < TE; j += 2) {
+                                const float2 sap = *reinterpret_cast<const float2 *>(sa + j);
+                                int i0 = (int)v[j], i1 = (int)v[j + 1];
+                                if (A_UNSIGNED) { i0 = (i0 >> 8) - za[j] * rsv[q]; i1 = (i1 >> 8) - za[j + 1] * rsv[q]; }
+                                const uint64_t p2 = mul2(pack2(sap.x, sap.y), sb2);
+                                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(accf[j >> 1]) : "l"(pack2((float)i0, (float)i1)), "l"(p2));
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < KP; ++q) { sbv[q] = nsb[q]; rsv[q] = nrs[q]; }
                 }
             } else {
                 const int buf = u % NBUF;
-                ok = __all_sync(0xffffffffu, ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 7, &w6));
+                ok = ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 7, &w6);
                 tc_fence_after();
                 uint32_t v[TE];
                 if (ok) { tmem_ld_cols<TE>(tlane + buf * TOK + j0, v); tc_wait_ld(); }
@@ -490,22 +523,23 @@ struct DecodeSplit { int tok, grid, per; };
 
 // Token columns, CTAs and K-blocks per CTA for a shape: as many CTAs as can be resident (two per SM up to 32
 // tokens, one above), never fewer than four K-blocks each unless the whole problem is smaller than that.
-DecodeSplit decode_split(long M, long N, long K) {
+DecodeSplit decode_split(long M, long N, long K, int kp = 1) {
     DecodeSplit d;
     d.tok = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     const long total = (N / BR) * (K / BK);
     const long slots = (long)sm_count() * (d.tok <= 32 ? 2 : 1);
     long per = (total + slots - 1) / slots;
     if (per < 4) per = total < 4 ? total : 4;
+    per = (per + kp - 1) / kp * kp;
     d.per = (int)per;
     d.grid = (int)((total + per - 1) / per);
     return d;
 }
 
-template <int TOK, bool G, bool U>
+template <int TOK, bool G, bool U, int KP>
 int launch_t(const CUtensorMap &mw, const CUtensorMap &mx, const DecParams &p, int grid, int aux_bytes, cudaStream_t stream) {
-    using Plan = DecPlan<TOK, G>;
-    auto kern = gemm_decode_tc_kernel<TOK, G, U>;
+    using Plan = DecPlan<TOK, G, KP>;
+    auto kern = gemm_decode_tc_kernel<TOK, G, U, KP>;
     const int smem = Plan::kAuxOff + aux_bytes + Plan::kSlack;
     if (smem > 227 * 1024) return fail(FLH_B200_EUNSUPPORTED, "K = %d needs %d bytes of shared memory for the token scales", p.K, smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -514,9 +548,11 @@ int launch_t(const CUtensorMap &mw, const CUtensorMap &mx, const DecParams &p, i
 }
 
 template <int TOK>
-int launch_tok(const CUtensorMap &mw, const CUtensorMap &mx, const DecParams &p, bool grouped, bool u, int grid, int aux, cudaStream_t s) {
-    if (grouped) return u ? launch_t<TOK, true, true>(mw, mx, p, grid, aux, s) : launch_t<TOK, true, false>(mw, mx, p, grid, aux, s);
-    return u ? launch_t<TOK, false, true>(mw, mx, p, grid, aux, s) : launch_t<TOK, false, false>(mw, mx, p, grid, aux, s);
+int launch_tok(const CUtensorMap &mw, const CUtensorMap &mx, const DecParams &p, bool grouped, bool u, int kp, int grid, int aux, cudaStream_t s) {
+    if constexpr (TOK == 64)
+        if (grouped && kp == 2) return launch_t<TOK, true, false, 2>(mw, mx, p, grid, aux, s);
+    if (grouped) return u ? launch_t<TOK, true, true, 1>(mw, mx, p, grid, aux, s) : launch_t<TOK, true, false, 1>(mw, mx, p, grid, aux, s);
+    return u ? launch_t<TOK, false, true, 1>(mw, mx, p, grid, aux, s) : launch_t<TOK, false, false, 1>(mw, mx, p, grid, aux, s);
 }
 
 }  // namespace
@@ -527,7 +563,8 @@ bool gemm_decode_tc_supported(long M, long N, long K, long a_group) {
     if (M < 1 || M > 64 || N % BR || K % BK || N / BR > kMaxTiles) return false;
     const int tok = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     const long aux = (a_group < K ? (K / BK) * tok : tok) * 8;      // with zero-points
-    const long fixed = tok == 16 ? DecPlan<16, true>::kAuxOff : (tok == 32 ? DecPlan<32, true>::kAuxOff : DecPlan<64, true>::kAuxOff);
+    const long fixed = tok == 16 ? DecPlan<16, true, 1>::kAuxOff : (tok == 32 ? DecPlan<32, true, 1>::kAuxOff : DecPlan<64, true, 1>::kAuxOff);
+    static_assert(DecPlan<64, true, 2>::kAuxOff <= DecPlan<64, true, 1>::kAuxOff, "a step of two K-blocks fits where one does");
     return fixed + aux + 1024 <= 227 * 1024;
 }
 
@@ -551,12 +588,14 @@ int launch_gemm_decode_tc(const uint8_t *A, const uint8_t *B, const void *a_scal
     p.M = (int)M; p.N = (int)N; p.K = (int)K; p.KB = (int)(K / BK);
     p.ga_cols = (int)(K / a_group); p.gb_cols = (int)(K / b_group);
     p.out_bf16 = out_dtype == FLH_B200_BF16;
-    const DecodeSplit d = decode_split(M, N, K);
+    const bool grouped = a_group < K || b_group < K;
+    // the workspace was sized for single K-blocks: ranges of two can only be fewer
+    const int kp = grouped && !a_zero && M > 32 && p.KB % 2 == 0 ? 2 : 1;
+    const DecodeSplit d = decode_split(M, N, K, kp);
     p.per = d.per;
     p.total = (int)((N / BR) * (K / BK));
     p.counters = static_cast<int *>(workspace);
     p.partials = reinterpret_cast<float *>(static_cast<uint8_t *>(workspace) + kCounterBytes);
-    const bool grouped = a_group < K || b_group < K;
     const bool u = a_zero != nullptr;
     const int aux = (p.ga_cols > 1 ? p.KB * d.tok : d.tok) * (u ? 8 : 4);
     const CUtensorMap *mw = nullptr, *mx = nullptr;
@@ -564,9 +603,9 @@ int launch_gemm_decode_tc(const uint8_t *A, const uint8_t *B, const void *a_scal
     if (rc) return rc;
     rc = get_map(g_maps_x, &mx, A, M, K, d.tok);
     if (rc) return rc;
-    if (d.tok == 16) return launch_tok<16>(*mw, *mx, p, grouped, u, d.grid, aux, stream);
-    if (d.tok == 32) return launch_tok<32>(*mw, *mx, p, grouped, u, d.grid, aux, stream);
-    return launch_tok<64>(*mw, *mx, p, grouped, u, d.grid, aux, stream);
+    if (d.tok == 16) return launch_tok<16>(*mw, *mx, p, grouped, u, kp, d.grid, aux, stream);
+    if (d.tok == 32) return launch_tok<32>(*mw, *mx, p, grouped, u, kp, d.grid, aux, stream);
+    return launch_tok<64>(*mw, *mx, p, grouped, u, kp, d.grid, aux, stream);
 }
 
 int gemm_decode_tc_status(int *out4) {
