@@ -19,6 +19,7 @@ SIGNATURES = {
     "flh_b200_last_error": (ctypes.c_char_p, []),
     "flh_b200_device_check": (c_int, []),
     "flh_b200_quant_group_sym_i4": (c_int, [c_void_p, c_long, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "flh_b200_quant_group_sym_scaled_i4": (c_int, [c_void_p, c_long, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p]),
     "flh_b200_hadamard_f16_inplace": (c_int, [c_void_p, c_long, c_int, c_void_p]),
     "flh_b200_quant_token_asym_i4": (c_int, [c_void_p, c_int, c_long, c_long, c_long, c_int, c_int, c_void_p, c_float,
                                              c_void_p, c_void_p, c_void_p, c_void_p]),

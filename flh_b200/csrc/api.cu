@@ -28,7 +28,7 @@ int cuda_status(cudaError_t e, const char *what) {
 }
 
 // kernels (other translation units)
-int launch_quant_group_sym(const void *, long, int, int, uint8_t *, void *, cudaStream_t);
+int launch_quant_group_sym(const void *, long, int, int, float, uint8_t *, void *, cudaStream_t);
 int launch_fht_inplace(void *, long, int, cudaStream_t);
 int launch_quant_token_asym(const void *, int, long, long, long, int, int, const uint32_t *, float,
                             uint8_t *, void *, void *, cudaStream_t);
@@ -134,13 +134,18 @@ int flh_b200_device_check(void) {
 
 int flh_b200_quant_group_sym_i4(const void *x, long rows, int gs, int hadamard, uint8_t *q,
                                 void *scales, void *stream) {
+    return flh_b200_quant_group_sym_scaled_i4(x, rows, gs, hadamard, 1.0f, q, scales, stream);
+}
+
+int flh_b200_quant_group_sym_scaled_i4(const void *x, long rows, int gs, int hadamard, float factor, uint8_t *q,
+                                       void *scales, void *stream) {
     FLH_REQUIRE(rows >= 0, FLH_B200_EINVAL, "rows must be >= 0 (got %ld)", rows);
     FLH_REQUIRE(gs == 32 || gs == 64 || gs == 128, FLH_B200_EINVAL, "group size must be 32, 64 or 128 (got %d)", gs);
     if (rows == 0) return 0;
     FLH_REQUIRE(x && q && scales, FLH_B200_EINVAL, "null pointer");
     FLH_REQUIRE(aligned16(x), FLH_B200_EALIGN, "x must be 16-byte aligned");
     FLH_REQUIRE((reinterpret_cast<uintptr_t>(q) & 3) == 0, FLH_B200_EALIGN, "q must be 4-byte aligned");
-    return launch_quant_group_sym(x, rows, gs, hadamard != 0, q, scales, static_cast<cudaStream_t>(stream));
+    return launch_quant_group_sym(x, rows, gs, hadamard != 0, factor, q, scales, static_cast<cudaStream_t>(stream));
 }
 
 int flh_b200_hadamard_f16_inplace(void *x, long rows, int n, void *stream) {

@@ -61,10 +61,11 @@ PyObject *act_quant_group(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const int64_t K = x->size(-1);
     if (!plain(*x, dev) || x->numel() == 0 || K % gs) Py_RETURN_NONE;
     at::Tensor q = empty(with_last(*x, K / 2), at::kByte, *x), s = empty(with_last(*x, K / gs), at::kHalf, *x);
-    const int rc = flh_b200_quant_group_sym_i4(x->data_ptr(), x->numel() / gs, (int)gs, had, static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(),
-                                               c10::cuda::getCurrentCUDAStream(dev).stream());
+    // torch divides a CUDA tensor by a number by multiplying with the number's reciprocal, rounded to binary32
+    const float factor = had ? 1.0f / (float)std::sqrt((double)gs) : 1.0f;
+    const int rc = flh_b200_quant_group_sym_scaled_i4(x->data_ptr(), x->numel() / gs, (int)gs, had, factor, static_cast<uint8_t *>(q.data_ptr()),
+                                                      s.data_ptr(), c10::cuda::getCurrentCUDAStream(dev).stream());
     if (rc) return failed("quant_group_sym_i4", rc);
-    if (had) s = at::div(s, at::Scalar(std::sqrt((double)gs)));
     return Py_BuildValue("(NN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)));
     END_HANDLE_TH_ERRORS
 }

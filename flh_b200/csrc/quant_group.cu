@@ -92,10 +92,16 @@ __device__ __forceinline__ uint32_t quant_pack8(const __half2 (&h)[4], float rcp
     return od * 16u + ev;
 }
 
+// the scale as it is handed out: times a factor of the caller's (the codes are made with the scale itself), rounded as a tensor
+// operation behind the kernel would round it; that operation is a launch of its own, 22 -> 16 -> 14 us with the host's part
+__device__ __forceinline__ __half scaled(__half s, float factor) {
+    return factor == 1.0f ? s : __float2half_rn(__fmul_rn(__half2float(s), factor));
+}
+
 template <int LOG_GS, bool HADAMARD>
 __global__ void __launch_bounds__(kThreads)
 quant_group_sym_kernel(const uint4 *__restrict__ x, uint32_t *__restrict__ q,
-                       __half *__restrict__ scales, long total_chunks) {
+                       __half *__restrict__ scales, long total_chunks, float factor) {
     constexpr int L = (1 << LOG_GS) / 8;          // lanes per group
     const long nthreads = (long)gridDim.x * kThreads;
     const long tid = (long)blockIdx.x * kThreads + threadIdx.x;
@@ -133,7 +139,7 @@ quant_group_sym_kernel(const uint4 *__restrict__ x, uint32_t *__restrict__ q,
             const uint32_t packed = quant_pack8(h, rcp);
             if (c < total_chunks) {
                 q[c] = packed;
-                if (lig == 0) scales[c / L] = sh;
+                if (lig == 0) scales[c / L] = scaled(sh, factor);
             }
         }
     }
@@ -177,7 +183,7 @@ __device__ __forceinline__ void stage_groups(const uint8_t *x, long tile, long t
 // rounded, y = half(x * c)).
 template <int GS, bool HADAMARD, bool NORM = false>
 __global__ void __launch_bounds__(kTWarps * 32, 4)
-quant_group_thread_kernel(const uint8_t *__restrict__ x, uint4 *__restrict__ q, __half *__restrict__ scales, long groups, float eps = 0.0f) {
+quant_group_thread_kernel(const uint8_t *__restrict__ x, uint4 *__restrict__ q, __half *__restrict__ scales, long groups, float eps, float factor) {
     static_assert(!NORM || GS == 128, "the fused norm is written for rows of 4096 = 32 groups of 128");
     constexpr int NH = GS / 2;                              // half2 registers of a group
     constexpr int kTile = 64 * GS;                          // bytes of one warp tile
@@ -257,7 +263,7 @@ quant_group_thread_kernel(const uint8_t *__restrict__ x, uint4 *__restrict__ q, 
                 }
                 q[g * (GS / 32) + v] = make_uint4(o[0], o[1], o[2], o[3]);
             }
-            scales[g] = sh;
+            scales[g] = scaled(sh, factor);
         }
     }
 }
@@ -325,7 +331,7 @@ static long group_thread_min_rows() {
     return v;
 }
 
-int launch_quant_group_sym(const void *x, long rows, int gs, int hadamard, uint8_t *q,
+int launch_quant_group_sym(const void *x, long rows, int gs, int hadamard, float factor, uint8_t *q,
                            void *scales, cudaStream_t stream) {
     const long chunks = rows * (gs / 8);
     // many groups of 128: the thread-per-group kernel (a full wave of its persistent warps has 32 groups each)
@@ -336,7 +342,7 @@ int launch_quant_group_sym(const void *x, long rows, int gs, int hadamard, uint8
         const uint8_t *xb = static_cast<const uint8_t *>(x);
         uint4 *qo4 = reinterpret_cast<uint4 *>(q);
         __half *so4 = static_cast<__half *>(scales);
-#define FLH_TLAUNCH(GS_, H_) e = launch_pdl(quant_group_thread_kernel<GS_, H_>, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * GS_, stream, xb, qo4, so4, rows, 0.0f)
+#define FLH_TLAUNCH(GS_, H_) e = launch_pdl(quant_group_thread_kernel<GS_, H_>, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * GS_, stream, xb, qo4, so4, rows, 0.0f, factor)
         cudaError_t e;
         if (gs == 128) { if (hadamard) FLH_TLAUNCH(128, true); else FLH_TLAUNCH(128, false); }
         else if (gs == 64) { if (hadamard) FLH_TLAUNCH(64, true); else FLH_TLAUNCH(64, false); }
@@ -347,7 +353,7 @@ int launch_quant_group_sym(const void *x, long rows, int gs, int hadamard, uint8
     const uint4 *xi = static_cast<const uint4 *>(x);
     uint32_t *qo = reinterpret_cast<uint32_t *>(q);
     __half *so = static_cast<__half *>(scales);
-#define FLH_LAUNCH(LG, H) e = launch_pdl(quant_group_sym_kernel<LG, H>, dim3(grid_for(quant_group_sym_kernel<LG, H>, chunks)), kThreads, 0, stream, xi, qo, so, chunks)
+#define FLH_LAUNCH(LG, H) e = launch_pdl(quant_group_sym_kernel<LG, H>, dim3(grid_for(quant_group_sym_kernel<LG, H>, chunks)), kThreads, 0, stream, xi, qo, so, chunks, factor)
     cudaError_t e;
     if (gs == 128) { if (hadamard) FLH_LAUNCH(7, true); else FLH_LAUNCH(7, false); }
     else if (gs == 64) { if (hadamard) FLH_LAUNCH(6, true); else FLH_LAUNCH(6, false); }
@@ -366,7 +372,7 @@ int launch_rmsnorm_quant_group(const void *x, long M, int hadamard, float eps, u
     uint4 *qo4 = reinterpret_cast<uint4 *>(q);
     __half *so4 = static_cast<__half *>(scales);
     const auto kern = hadamard ? quant_group_thread_kernel<128, true, true> : quant_group_thread_kernel<128, false, true>;
-    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * 128, stream, xb, qo4, so4, groups, eps), "rmsnorm_quant_group launch");
+    return cuda_status(launch_pdl(kern, dim3((unsigned)grid), kTWarps * 32, kTWarps * 64 * 128, stream, xb, qo4, so4, groups, eps, 1.0f), "rmsnorm_quant_group launch");
 }
 
 int launch_fht_inplace(void *x, long rows, int n, cudaStream_t stream) {

@@ -81,6 +81,11 @@ int flh_b200_device_check(void);
 int flh_b200_quant_group_sym_i4(const void *x, long rows, int gs, int hadamard,
                                 uint8_t *q, void *scales, void *stream);
 
+/* The same with every scale multiplied by `factor` as it is written (binary32 product of the f16 scale, rounded to f16): the
+ * scales of the normalised transform with factor = 1 / sqrt(gs).  The codes do not depend on it. */
+int flh_b200_quant_group_sym_scaled_i4(const void *x, long rows, int gs, int hadamard, float factor, uint8_t *q,
+                                       void *scales, void *stream);
+
 /* In-place un-normalised f16 Walsh-Hadamard transform of rows of n in {32, 64, 128}.
  * Replaces had_trans_half_cuda / had_trans_64_half_cuda / had_trans_32_half_cuda
  * (flh/kernels/cuda_had_kernel.cu:296-354 and the 64/32 copies), bound as

@@ -70,6 +70,18 @@ def test_quantiser_native_equals_python(cuda, monkeypatch, k, sym, group, had, d
         assert _same(native, plain), (tuple(x.shape), x.dtype, x.device, native, plain)
 
 
+@pytest.mark.parametrize("gs", [32, 64, 128])
+def test_scales_of_the_normalised_transform(cuda, monkeypatch, gs):
+    """Every size a scale can have: the factor inside the kernel rounds as torch's division behind it."""
+    x = torch.zeros(65536, gs, dtype=torch.float16, device="cuda")
+    x[:, 0] = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.float16)     # an impulse: all group values are it
+    quant = ActQuantizer(bits=4, group_size=gs, sym=True, use_hadamard=True, packed_output=True)
+    for rows in (65536, 100):                            # the kernel of many groups, the kernel of few
+        (s, _, q), (s2, _, q2) = quant(x[:rows]), (monkeypatch.setattr(cuda, "_host", None), quant(x[:rows]))[1]
+        monkeypatch.undo()
+        assert torch.equal(s.view(torch.int16), s2.view(torch.int16)) and torch.equal(q, q2)
+
+
 @pytest.mark.parametrize("m", [1, 16, 64, 130])
 @pytest.mark.parametrize("group,zero,bias,out", [(128, False, False, None), (128, False, True, torch.bfloat16), (-1, True, True, None), (-1, False, False, torch.bfloat16)])
 def test_linear_native_equals_python(cuda, monkeypatch, m, group, zero, bias, out):
