@@ -6,6 +6,10 @@
 // Every function takes the plain case only and returns None for anything else — another type, layout or device than the
 // current one, a tensor subclass, a transform, mode or trace that has to see the operations — and the caller then goes the
 // way in Python, which has the error messages and the general shapes.  Nothing is kept between calls.
+//
+// Allocations and launches run without the interpreter's lock: an allocation may free blocks and synchronise, and a launch waits
+// while the stream's queue is full, for as long as the GPU takes; other Python threads run meanwhile, among them the one that
+// what is queued may be waiting for.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -35,6 +39,14 @@ bool plain(const at::Tensor &t, c10::DeviceIndex device) {
 }
 const at::Tensor *tensor(PyObject *o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
 
+// the interpreter's lock given up for a scope, taken back also where an exception leaves it
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked &) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 PyObject *failed(const char *what, int rc) {
     PyErr_Format(PyExc_RuntimeError, "%s failed (status %d): %s", what, rc, flh_b200_last_error());
     return nullptr;
@@ -60,11 +72,19 @@ PyObject *act_quant_group(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const c10::DeviceIndex dev = c10::cuda::current_device();
     const int64_t K = x->size(-1);
     if (!plain(*x, dev) || x->numel() == 0 || K % gs) Py_RETURN_NONE;
-    at::Tensor q = empty(with_last(*x, K / 2), at::kByte, *x), s = empty(with_last(*x, K / gs), at::kHalf, *x);
+    const at::Tensor in = *x;
+    const void *in_p = in.data_ptr();
+    at::Tensor q, s;
+    int rc;
     // torch divides a CUDA tensor by a number by multiplying with the number's reciprocal, rounded to binary32
     const float factor = had ? 1.0f / (float)std::sqrt((double)gs) : 1.0f;
-    const int rc = flh_b200_quant_group_sym_scaled_i4(x->data_ptr(), x->numel() / gs, (int)gs, had, factor, static_cast<uint8_t *>(q.data_ptr()),
-                                                      s.data_ptr(), c10::cuda::getCurrentCUDAStream(dev).stream());
+    {
+        const Unlocked unlocked;
+        q = empty(with_last(in, K / 2), at::kByte, in);
+        s = empty(with_last(in, K / gs), at::kHalf, in);
+        rc = flh_b200_quant_group_sym_scaled_i4(in_p, in.numel() / gs, (int)gs, had, factor, static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(),
+                                                c10::cuda::getCurrentCUDAStream(dev).stream());
+    }
     if (rc) return failed("quant_group_sym_i4", rc);
     return Py_BuildValue("(NN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)));
     END_HANDLE_TH_ERRORS
@@ -83,13 +103,22 @@ PyObject *act_quant_token(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16) Py_RETURN_NONE;
     const c10::DeviceIndex dev = c10::cuda::current_device();
     if (!plain(*x, dev) || x->numel() == 0) Py_RETURN_NONE;
-    const int64_t K = x->size(-1);
-    const auto one = with_last(*x, 1);
-    at::Tensor q = empty(with_last(*x, K / 2), at::kByte, *x), s = empty(one, at::kHalf, *x), z = empty(one, at::kHalf, *x);
-    const int rc = flh_b200_quant_token_asym_i4(x->data_ptr(), x->scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, x->numel() / K, K, K,
-                                                had ? 1 : 0, (int)kfac, bits ? static_cast<const uint32_t *>(bits->data_ptr()) : nullptr, (float)clip,
-                                                static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(), z.data_ptr(),
-                                                c10::cuda::getCurrentCUDAStream(dev).stream());
+    const at::Tensor in = *x, table = bits ? *bits : at::Tensor();
+    const void *in_p = in.data_ptr();
+    const uint32_t *table_p = bits ? static_cast<const uint32_t *>(table.data_ptr()) : nullptr;
+    const int64_t K = in.size(-1);
+    at::Tensor q, s, z;
+    int rc;
+    {
+        const Unlocked unlocked;
+        const auto one = with_last(in, 1);
+        q = empty(with_last(in, K / 2), at::kByte, in);
+        s = empty(one, at::kHalf, in);
+        z = empty(one, at::kHalf, in);
+        rc = flh_b200_quant_token_asym_i4(in_p, in.scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, in.numel() / K, K, K, had ? 1 : 0,
+                                          (int)kfac, table_p, (float)clip, static_cast<uint8_t *>(q.data_ptr()), s.data_ptr(), z.data_ptr(),
+                                          c10::cuda::getCurrentCUDAStream(dev).stream());
+    }
     if (rc) return failed("quant_token_asym_i4", rc);
     return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(q)), THPVariable_Wrap(std::move(s)), THPVariable_Wrap(std::move(z)));
     END_HANDLE_TH_ERRORS
@@ -124,20 +153,32 @@ PyObject *gemm(PyObject *, PyObject *const *args, Py_ssize_t n) {
         sb.scalar_type() != at::kHalf || (t[3] && (t[3]->scalar_type() != at::kHalf || t[3]->numel() != sa.numel())) ||
         (t[5] && t[5]->scalar_type() != at::kInt) || (t[6] && (t[6]->scalar_type() != at::kHalf || t[6]->numel() != N)))
         Py_RETURN_NONE;
-    at::Tensor y = empty(with_last(x, N), bf16 ? at::kBFloat16 : at::kHalf, x), own;
-    if (scratch > 0) {
-        try {
-            own = empty({(int64_t)scratch}, at::kByte, x);       // freed in stream order when the call returns
-        } catch (const c10::OutOfMemoryError &) {
-            Py_RETURN_NONE;                                      // AUTO has a kernel that needs none
+    at::Tensor held[8], y, own;                                  // the operands and the workspace stay alive while the lock is given up
+    void *ptr[8] = {};
+    for (int i = 0; i < 7; ++i)
+        if (t[i]) { held[i] = *t[i]; ptr[i] = t[i]->data_ptr(); }
+    size_t ws_bytes = 0;
+    if (ws) { held[7] = *ws; ptr[7] = ws->data_ptr(); ws_bytes = (size_t)ws->numel(); }
+    int rc;
+    bool fits = true;
+    {
+        const Unlocked unlocked;
+        y = empty(with_last(held[0], N), bf16 ? at::kBFloat16 : at::kHalf, held[0]);
+        if (scratch > 0) {
+            try {
+                own = empty({(int64_t)scratch}, at::kByte, held[0]);     // freed in stream order when the call returns
+                ptr[7] = own.data_ptr();
+                ws_bytes = (size_t)scratch;
+            } catch (const c10::OutOfMemoryError &) {
+                fits = false;                                    // AUTO has a kernel that needs none
+            }
         }
-        ws = &own;
+        rc = !fits ? 0 : flh_b200_gemm_i4_dequant(
+            static_cast<const uint8_t *>(ptr[0]), static_cast<const uint8_t *>(ptr[1]), ptr[2], ptr[3], ptr[4], static_cast<const int32_t *>(ptr[5]),
+            ptr[6], y.data_ptr(), M, N, K, K / ga, K / gb, bf16 ? FLH_B200_BF16 : FLH_B200_F16, (int)algo, ptr[7], ws_bytes,
+            c10::cuda::getCurrentCUDAStream(dev).stream());
     }
-    const int rc = flh_b200_gemm_i4_dequant(
-        static_cast<const uint8_t *>(x.data_ptr()), static_cast<const uint8_t *>(w.data_ptr()), sa.data_ptr(), t[3] ? t[3]->data_ptr() : nullptr,
-        sb.data_ptr(), t[5] ? static_cast<const int32_t *>(t[5]->data_ptr()) : nullptr, t[6] ? t[6]->data_ptr() : nullptr, y.data_ptr(), M, N, K,
-        K / ga, K / gb, bf16 ? FLH_B200_BF16 : FLH_B200_F16, (int)algo, ws ? ws->data_ptr() : nullptr, ws ? (size_t)ws->numel() : 0,
-        c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (!fits) Py_RETURN_NONE;
     if (rc) return failed("gemm_i4_dequant", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
@@ -151,9 +192,16 @@ PyObject *square(PyObject *, PyObject *x_) {
     const c10::DeviceIndex dev = c10::cuda::current_device();
     if (!plain(*x, dev) || x->numel() % 8 || reinterpret_cast<uintptr_t>(x->data_ptr()) % 16) Py_RETURN_NONE;
     if ((c10::GradMode::is_enabled() && x->requires_grad()) || x->_fw_grad(0).defined()) Py_RETURN_NONE;
-    at::Tensor y = empty(x->sizes(), at::kFloat, *x);
-    const int rc = flh_b200_square_f32(x->data_ptr(), x->scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, x->numel(), y.data_ptr(),
-                                       c10::cuda::getCurrentCUDAStream(dev).stream());
+    const at::Tensor in = *x;
+    const void *in_p = in.data_ptr();
+    at::Tensor y;
+    int rc;
+    {
+        const Unlocked unlocked;
+        y = empty(in.sizes(), at::kFloat, in);
+        rc = flh_b200_square_f32(in_p, in.scalar_type() == at::kBFloat16 ? FLH_B200_BF16 : FLH_B200_F16, in.numel(), y.data_ptr(),
+                                 c10::cuda::getCurrentCUDAStream(dev).stream());
+    }
     if (rc) return failed("square_f32", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS

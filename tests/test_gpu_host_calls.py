@@ -1,5 +1,8 @@
 """The native form of the quantiser and linear calls (csrc/host_calls.cpp) against the way in Python: the same bits where it takes
 the arguments, the same results and errors where it leaves them to Python."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -109,3 +112,44 @@ def test_linear_native_equals_python(cuda, monkeypatch, m, group, zero, bias, ou
     y.zero_()
     graph.replay()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("what", ["group", "token", "linear", "squares"])
+def test_other_threads_run_while_a_call_waits_for_the_queue(cuda, what):
+    """Calls behind a kernel of half a second fill the stream's queue (1,024 launches), and the next one waits until that kernel is
+    done: meanwhile another thread keeps running.  Its longest pause is bounded by half of the whole time; the interpreter's lock held
+    through the wait makes it nearly all of that (what else pauses it is a few switch intervals of 5 ms)."""
+    k = 1024
+    x = torch.randn(1, 1, k, device="cuda").half()
+    packed = torch.randint(0, 256, (1, k // 2), dtype=torch.uint8, device="cuda")
+    scale = torch.ones(1, 1, device="cuda", dtype=torch.float16)
+    lin = LinearFLH(k, 128, dtype=torch.float16, device="cuda", group_size=-1)
+    group = ActQuantizer(bits=4, group_size=128, sym=True, use_hadamard=False, packed_output=True)
+    token = ActQuantizer(bits=4, group_size=-1, sym=False, use_hadamard=False, packed_output=True)
+    call = {"group": lambda: group(x), "token": lambda: token(x), "linear": lambda: lin(packed, scale), "squares": lambda: cuda.square_f32(x)}[what]
+    call()
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    ticks, stop = [time.perf_counter()], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.001)
+
+    other = threading.Thread(target=tick)
+    other.start()
+    try:
+        start = time.perf_counter()
+        torch.cuda._sleep(1_000_000_000)             # clocks
+        for _ in range(4000):
+            call()
+        torch.cuda.synchronize()
+        end = time.perf_counter()
+    finally:
+        stop.set()
+        other.join()
+    ticks.append(end)
+    pause = max(t1 - t0 for t0, t1 in zip(ticks, ticks[1:]))
+    assert end - start > 0.3
+    assert pause < 0.5 * (end - start), (pause, end - start)
