@@ -266,8 +266,9 @@ def act_quant_token(x, hadamard: bool, clip: float):
 
 def square_f32(x):
     """x * x in binary32, the bits of x.float().pow(2), in one pass: x a contiguous CUDA float16 or bfloat16 tensor whose numel is a
-    multiple of 8 and of which no derivative is taken; None for anything else."""
-    return None if _host is None else _host.square(x)
+    multiple of 8 and of which no derivative is taken; None for anything else, and while torch.compile or torch.export reads the
+    program: the compiler refuses a call that it cannot trace, and traces the tensor operations that stand for this one."""
+    return None if _host is None or torch.compiler.is_compiling() else _host.square(x)
 
 
 def silu_mul(gu):

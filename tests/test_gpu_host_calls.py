@@ -153,3 +153,28 @@ def test_other_threads_run_while_a_call_waits_for_the_queue(cuda, what):
     pause = max(t1 - t0 for t0, t1 in zip(ticks, ticks[1:]))
     assert end - start > 0.3
     assert pause < 0.5 * (end - start), (pause, end - start)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_final_norm_compiled_traced_and_transformed(cuda, dtype):
+    """What has to see the operations of the last position's norm sees them: the results are those of the whole norm."""
+    from flh_b200.model import RMSNorm
+
+    class Last(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.norm = RMSNorm(256, 1e-5).cuda()
+
+        def forward(self, x):
+            return self.norm(x, last=True)
+
+    norm, (x, t) = Last(), torch.randn(2, 2, 3, 256, device="cuda").to(dtype)
+    want = norm.norm(x)[:, -1:]
+    torch._dynamo.reset()
+    assert torch.equal(torch.compile(norm, fullgraph=True, backend="eager")(x), want)
+    assert torch.equal(torch.export.export(norm, (x,), strict=True).module()(x), want)
+    assert torch.equal(torch.jit.trace(norm, (t,), check_trace=False)(x), want)
+    assert torch.equal(torch.vmap(norm)(x[None])[0], want)
+    y, dy = torch.func.jvp(norm, (x,), (t,))
+    dw = torch.func.jvp(norm.norm, (x,), (t,))[1][:, -1:]
+    assert torch.equal(y, want) and torch.equal(dy, dw) and bool(dy.any())

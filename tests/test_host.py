@@ -149,3 +149,25 @@ def test_oracle_rmsnorm_matches_torch():
         yt = (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5)).half().float().numpy()
         assert np.all(np.abs(y - yt) <= np.maximum(np.abs(yt), 1e-3) * 2.0 ** -10)
         assert (y != yt).mean() < 1e-2
+
+
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("how", ["compile", "export"])
+def test_norm_is_compiled_and_exported_whole(how, last):
+    from flh_b200.model import RMSNorm
+
+    class Norm(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.norm = RMSNorm(64, 1e-5)
+
+        def forward(self, x):
+            return self.norm(x, last=last)
+
+    x, norm = torch.randn(2, 3, 64), Norm()
+    torch._dynamo.reset()
+    if how == "compile":
+        got = torch.compile(norm, fullgraph=True, backend="eager")(x)
+    else:
+        got = torch.export.export(norm, (x,), strict=True).module()(x)
+    assert torch.equal(got, norm(x))
