@@ -30,7 +30,8 @@ namespace {
 bool observed() {
     return at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() || torch::jit::tracer::isTracing();
 }
-// a contiguous CUDA tensor on `device` with memory of its own kind and nothing wrapped around it
+// a contiguous CUDA tensor on `device` (the current one, which is asked for only once a tensor is known to be a CUDA tensor: there may
+// be no driver) with memory of its own kind and nothing wrapped around it
 bool plain(const at::Tensor &t, c10::DeviceIndex device) {
     if (!t.is_cuda() || t.device().index() != device || t.layout() != at::kStrided || !t.is_contiguous() || t.is_neg() || t.is_conj()) return false;
     const c10::DispatchKeySet ks = t.key_set();
@@ -68,7 +69,7 @@ PyObject *act_quant_group(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const long gs = x ? PyLong_AsLong(args[1]) : 0;
     const int had = x ? PyObject_IsTrue(args[2]) : 0;
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (!x || observed() || (gs != 32 && gs != 64 && gs != 128) || x->dim() < 1 || x->scalar_type() != at::kHalf) Py_RETURN_NONE;
+    if (!x || !x->is_cuda() || observed() || (gs != 32 && gs != 64 && gs != 128) || x->dim() < 1 || x->scalar_type() != at::kHalf) Py_RETURN_NONE;
     const c10::DeviceIndex dev = c10::cuda::current_device();
     const int64_t K = x->size(-1);
     if (!plain(*x, dev) || x->numel() == 0 || K % gs) Py_RETURN_NONE;
@@ -99,7 +100,7 @@ PyObject *act_quant_token(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const double clip = x ? PyFloat_AsDouble(args[2]) : 0;
     const long kfac = x ? PyLong_AsLong(args[3]) : 0;
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (!x || (!bits && args[4] != Py_None) || observed() || x->dim() < 1) Py_RETURN_NONE;
+    if (!x || !x->is_cuda() || (!bits && args[4] != Py_None) || observed() || x->dim() < 1) Py_RETURN_NONE;
     if (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16) Py_RETURN_NONE;
     const c10::DeviceIndex dev = c10::cuda::current_device();
     if (!plain(*x, dev) || x->numel() == 0) Py_RETURN_NONE;
@@ -142,6 +143,7 @@ PyObject *gemm(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
     if ((!ws && !PyLong_Check(args[9]) && args[9] != Py_None) || observed()) Py_RETURN_NONE;
     const at::Tensor &x = *t[0], &w = *t[1], &sa = *t[2], &sb = *t[4];
+    if (!x.is_cuda()) Py_RETURN_NONE;
     const c10::DeviceIndex dev = c10::cuda::current_device();
     for (int i = 0; i < 7; ++i)
         if (t[i] && !plain(*t[i], dev)) Py_RETURN_NONE;
@@ -188,7 +190,7 @@ PyObject *gemm(PyObject *, PyObject *const *args, Py_ssize_t n) {
 PyObject *square(PyObject *, PyObject *x_) {
     HANDLE_TH_ERRORS
     const at::Tensor *x = tensor(x_);
-    if (!x || observed() || (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16)) Py_RETURN_NONE;
+    if (!x || !x->is_cuda() || observed() || (x->scalar_type() != at::kHalf && x->scalar_type() != at::kBFloat16)) Py_RETURN_NONE;
     const c10::DeviceIndex dev = c10::cuda::current_device();
     if (!plain(*x, dev) || x->numel() % 8 || reinterpret_cast<uintptr_t>(x->data_ptr()) % 16) Py_RETURN_NONE;
     if ((c10::GradMode::is_enabled() && x->requires_grad()) || x->_fw_grad(0).defined()) Py_RETURN_NONE;

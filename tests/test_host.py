@@ -171,3 +171,15 @@ def test_norm_is_compiled_and_exported_whole(how, last):
     else:
         got = torch.export.export(norm, (x,), strict=True).module()(x)
     assert torch.equal(got, norm(x))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_cpu_tensors_do_not_need_a_driver(dtype):
+    """The norm takes tensors of the host, the quantisers refuse them in their own words; neither asks for a device."""
+    from flh_b200.model import RMSNorm
+    from flh_b200.nn import ActQuantizer
+    norm, x = RMSNorm(64, 1e-5), torch.randn(2, 3, 64).to(dtype)
+    assert torch.equal(norm(x, last=True), norm(x)[:, -1:])
+    for sym in (True, False):
+        with pytest.raises(RuntimeError, match="Input tensor must be on CUDA"):
+            ActQuantizer(bits=4, group_size=32 if sym else -1, sym=sym, packed_output=True)(x)
