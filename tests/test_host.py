@@ -183,3 +183,17 @@ def test_cpu_tensors_do_not_need_a_driver(dtype):
     for sym in (True, False):
         with pytest.raises(RuntimeError, match="Input tensor must be on CUDA"):
             ActQuantizer(bits=4, group_size=32 if sym else -1, sym=sym, packed_output=True)(x)
+
+
+@pytest.mark.parametrize("compiler", ["false", "no-such-compiler"])
+def test_library_is_built_where_the_extension_cannot_be(monkeypatch, tmp_path, compiler):
+    from flh_b200 import build as b
+    host = tmp_path / "_host.so"
+    host.write_text("an older one")
+    monkeypatch.setattr(b, "SOURCES", [])                 # nothing of the library is stale
+    monkeypatch.setattr(b, "HOST", str(host))
+    monkeypatch.setattr(b, "_stale", lambda target, deps: target == str(host))
+    monkeypatch.setenv("CXX", compiler)
+    with pytest.warns(UserWarning, match=compiler):
+        assert b.build() == b.LIB
+    assert not host.exists()
