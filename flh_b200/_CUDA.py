@@ -13,17 +13,36 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import functools
+import importlib.util
 import math
+import warnings
 
 import numpy as np
 import torch
 
 from . import _lib
 from .hadamard import get_hadK
-try:
-    from . import _host         # csrc/host_calls.cpp: the same calls with less host time; built by `python -m flh_b200.build`
-except ImportError:             # not built yet, or a torch without CUDA
-    _host = None
+
+
+def _native_calls():
+    """csrc/host_calls.cpp, the same calls with less host time, or None: silently where it is not there (not built, or a torch without
+    CUDA), with a warning where it is there and of no use."""
+    name = __package__ + "._host"
+    if importlib.util.find_spec(name) is None:
+        return None
+    try:
+        module = importlib.import_module(name)
+        built_for = getattr(module, "torch_version", "another version")
+        why = None if built_for == torch.__version__ else f"it was built for torch {built_for}, this is {torch.__version__}"
+    except ImportError as e:
+        why = str(e)
+    if why is None:
+        return module
+    warnings.warn(f"{name} is not used, small calls take twice the host time (python -m flh_b200.build): {why}")
+    return None
+
+
+_host = _native_calls()
 
 F16, BF16 = 0, 1
 GEMM_AUTO, GEMM_TCGEN05, GEMM_MMA_SYNC, GEMM_STREAM, GEMM_STREAM_SPLITK, GEMM_TCGEN05_DIRECT = 0, 1, 2, 3, 4, 5

@@ -12,6 +12,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 import warnings
 from concurrent.futures import ThreadPoolExecutor
 
@@ -19,7 +20,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SOURCES = ["api.cu", "quant_group.cu", "quant_token.cu", "quant_token_warp.cu", "quant_token_factor.cu", "quant_token_tc.cu", "act.cu", "gemm_mma.cu", "gemm_tcgen05.cu", "gemm_i8.cu", "gemm_group_f8.cu", "gemm_decode_tc.cu", "gemm_decode_ring.cu", "gptq.cu", "allreduce.cu"]
 LIB = os.path.join(HERE, "libflh_b200.so")
-HOST = os.path.join(HERE, "_host.so")             # csrc/host_calls.cpp: the per-call host work as a Python extension on torch
+# csrc/host_calls.cpp: the per-call host work as a Python extension.  It is compiled against one CPython (the file's suffix) and one
+# torch, whose version is kept beside the objects and in the extension itself.
+HOST = os.path.join(HERE, "_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+HOST_TORCH = os.path.join(HERE, "build", "_host.torch")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
@@ -67,21 +71,31 @@ def build(verbose: bool = False, force: bool = False) -> str:
 
 
 def _build_host(run, force: bool) -> None:
+    import torch
     src = os.path.join(CSRC, "host_calls.cpp")
-    if not force and not _stale(HOST, [src, os.path.join(HERE, "..", "include", "flh_b200.h")]):
+    if not force and not _stale(HOST, [src, os.path.join(HERE, "..", "include", "flh_b200.h")]) and _built_for() == torch.__version__:
         return
     if os.path.exists(HOST):
         os.remove(HOST)                             # what does not build again is not loaded
-    import sysconfig
-    import torch
     from torch.utils import cpp_extension
     if torch.version.cuda is None:
         return                                      # nothing to launch on: flh_b200/_CUDA.py does without
     include = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cpp_extension.CUDA_HOME or "/usr/local/cuda", "include")]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DFLH_TORCH="{torch.__version__}"',
          *[f"-I{i}" for i in include], src, "-o", HOST, f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_cuda",
          "-ltorch_python", f"-L{HERE}", "-l:libflh_b200.so", "-Wl,-rpath,$ORIGIN"])
+    with open(HOST_TORCH, "w") as f:
+        f.write(torch.__version__)
+
+
+def _built_for():
+    """The torch version that HOST was compiled against, or None."""
+    try:
+        with open(HOST_TORCH) as f:
+            return f.read()
+    except OSError:
+        return None
 
 
 if __name__ == "__main__":

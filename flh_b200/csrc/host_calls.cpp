@@ -219,4 +219,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+// torch_version: what the tensors' layout was compiled against; flh_b200/_CUDA.py uses the module under that version only
+PyMODINIT_FUNC PyInit__host(void) {
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_version", FLH_TORCH) < 0) { Py_DECREF(m); return nullptr; }
+    return m;
+}

@@ -197,3 +197,35 @@ def test_library_is_built_where_the_extension_cannot_be(monkeypatch, tmp_path, c
     with pytest.warns(UserWarning, match=compiler):
         assert b.build() == b.LIB
     assert not host.exists()
+
+
+def test_extension_of_another_torch_is_built_again_and_not_used(monkeypatch, tmp_path):
+    from flh_b200 import _CUDA, build as b
+    assert b._built_for() == torch.__version__ == _CUDA._native_calls().torch_version
+    monkeypatch.setattr(b, "SOURCES", [])
+    monkeypatch.setattr(b, "HOST", str(tmp_path / "_host.so"))
+    (tmp_path / "_host.so").write_text("")
+    monkeypatch.setattr(b, "HOST_TORCH", str(tmp_path / "version"))
+    monkeypatch.setattr(b, "_stale", lambda target, deps: False)
+    monkeypatch.setenv("CXX", "true")
+    for version, again in (("0.0", True), (None, False)):      # and then the version that was just written down
+        if version is not None:
+            (tmp_path / "version").write_text(version)
+        (tmp_path / "_host.so").write_text("")
+        b.build()
+        assert (tmp_path / "_host.so").exists() is not again and (tmp_path / "version").read_text() == torch.__version__
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    with pytest.warns(UserWarning, match="built for torch"):
+        assert _CUDA._native_calls() is None
+
+
+def test_extension_that_does_not_load_is_reported(monkeypatch):
+    from flh_b200 import _CUDA
+
+    def broken(name):
+        raise ImportError("undefined symbol")
+    monkeypatch.setattr(_CUDA.importlib, "import_module", broken)
+    with pytest.warns(UserWarning, match="undefined symbol"):
+        assert _CUDA._native_calls() is None
+    monkeypatch.setattr(_CUDA.importlib.util, "find_spec", lambda name: None)        # not built: nothing to report
+    assert _CUDA._native_calls() is None
