@@ -79,10 +79,15 @@ def test_scales_of_the_normalised_transform(cuda, monkeypatch, gs):
     x = torch.zeros(65536, gs, dtype=torch.float16, device="cuda")
     x[:, 0] = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.float16)     # an impulse: all group values are it
     quant = ActQuantizer(bits=4, group_size=gs, sym=True, use_hadamard=True, packed_output=True)
-    for rows in (65536, 100):                            # the kernel of many groups, the kernel of few
-        (s, _, q), (s2, _, q2) = quant(x[:rows]), (monkeypatch.setattr(cuda, "_host", None), quant(x[:rows]))[1]
+    parts = [x, *x.split(2048)]                          # the kernel of many groups; the kernel of few, which the same values reach in parts
+    seen = set()
+    for part in parts:
+        (s, _, q), (s2, _, q2) = quant(part), (monkeypatch.setattr(cuda, "_host", None), quant(part))[1]
         monkeypatch.undo()
         assert torch.equal(s.view(torch.int16), s2.view(torch.int16)) and torch.equal(q, q2)
+        if part is not x:
+            seen.update(s.view(torch.int16).unique().tolist())
+    assert len(seen) > 10000                             # most are no floor
 
 
 @pytest.mark.parametrize("m", [1, 16, 64, 130])
