@@ -39,13 +39,16 @@ __device__ int g_status[4];
 // [6] epilogue on acc_full, [7] epilogue in the arrival protocol of shared tiles.  Diagnostic only.
 __device__ unsigned long long g_wait_ns[8];
 
+// VOTE: by a whole warp, with one outcome for all its lanes; otherwise each lane's own.  A try may already sleep in hardware, so what
+// does not succeed at once is timed as a whole.
+template <bool VOTE>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int code,
                                           unsigned long long *waited = nullptr) {
-    // by whole warps, with one outcome for all lanes; a try may already sleep in hardware, so what does not succeed at once is timed
-    // as a whole
-    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    const bool there = mbar_test(bar, parity);
+    if (VOTE ? (bool)__all_sync(0xffffffffu, there) : there) return true;
     const uint64_t t0 = waited ? gtimer() : 0;
-    const bool ok = __all_sync(0xffffffffu, mbar_wait_status(g_status, bar, parity, abort_flag, code));
+    bool ok = mbar_wait_status(g_status, bar, parity, abort_flag, code);
+    if (VOTE) ok = __all_sync(0xffffffffu, ok);
     if (waited) *waited += gtimer() - t0;
     return ok;
 }
@@ -102,6 +105,20 @@ __global__ void __launch_bounds__((DecPlan<TOK, GROUPED, KP>::kThreads), TOK <= 
 gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                       const DecParams p) {
     using Plan = DecPlan<TOK, GROUPED, KP>;
+    // How the roles walk their loops and meet, each where it measured faster (B200, us, weights from HBM).
+    //   VOTE   waits with one outcome for the warp: the steps of two K-blocks only.  64 tokens, per-token scales, 8192 -> 10240: 25.4 with
+    //          the vote, 24.7 without.
+    //   SOLO   TMA and MMA loops walked by one lane in place of the warp with one lane elected: without group scales, and 32 tokens with
+    //          group scales and zero-points.  64 tokens, per-token scales, 8192 -> 57344: 80.4 / 82.1 by the warp, 32 tokens
+    //          28672 -> 8192 36.4 / 38.0; 32 tokens with group scales 8192 -> 28672 55.0 / 53.1 the other way round.
+    //   LANES  every lane arrives in place of one for its warp, where two CTAs share the SM, but not 16 tokens with group scales.
+    //          32 tokens with group scales 28672 -> 8192 71.9 / 74.8, with zero-points 8192 -> 57344 146.5 / 157.6; 16 tokens, per-token
+    //          scales, 11008 -> 4096 15.5 / 15.9; 64 tokens 85.8 / 80.4 the other way round.
+    constexpr bool VOTE = KP == 2, LANES = TOK <= 32 && !(TOK == 16 && GROUPED);
+    constexpr bool SOLO = KP == 1 && (!GROUPED || (TOK == 32 && A_UNSIGNED));
+    auto uniform = [](bool ok) { return VOTE ? ok : (bool)__all_sync(0xffffffffu, ok); };
+    auto uniform_issue = [](bool ok) { return VOTE || SOLO ? ok : (bool)__all_sync(0xffffffffu, ok); };
+    auto meet = []() { if (!LANES) __syncwarp(); };      // in front of an arrival
     constexpr int SP = Plan::SP, SE = Plan::SE, NBUF = Plan::NBUF, EG = Plan::EG, TE = TOK / EG;
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t raw = smem_u32(smem_dyn);
@@ -133,10 +150,12 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     float *sa_s = reinterpret_cast<float *>(sm + Plan::kAuxOff);
     int *za_s = reinterpret_cast<int *>(sa_s + sa_n);
 
+    constexpr int kArrive = LANES ? 128 : 4;         // arrivals of four warps
+    const bool arrives = LANES || lane == 0;
     if (tid == 0) {
-        for (int s = 0; s < SP; ++s) { mbar_init(pk_full(s), 1); mbar_init(pk_empty(s), 4); }
-        for (int s = 0; s < SE; ++s) { mbar_init(ex_full(s), 4); mbar_init(ex_empty(s), 1); }
-        for (int b = 0; b < NBUF; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4 * EG); }
+        for (int s = 0; s < SP; ++s) { mbar_init(pk_full(s), 1); mbar_init(pk_empty(s), kArrive); }
+        for (int s = 0; s < SE; ++s) { mbar_init(ex_full(s), kArrive); mbar_init(ex_empty(s), 1); }
+        for (int b = 0; b < NBUF; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), kArrive * EG); }
         *abort_flag = 0;
         s_last[0] = 0; s_last[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -153,71 +172,75 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     pdl_wait();                                     // the set-up overlaps the kernel that makes the tokens
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        int tile = lin_begin / KB, kb = lin_begin - tile * KB;
-        int it = 0, s = 0;
-        uint32_t ph = 1;
-        unsigned long long w1 = 0;
-        for (; it < steps; ++it) {
-            if (!mbar_wait(pk_empty(s), ph, abort_flag, 1, &w1)) break;
-            const uint32_t dst = base + Plan::kPkOff + s * Plan::kPkStage;
-            if (elect_one()) {
-                mbar_expect_tx(pk_full(s), Plan::kPkStage);
+        if (!SOLO || lane == 0) {
+            // ------------------------------------------------------------ TMA producer
+            int tile = lin_begin / KB, kb = lin_begin - tile * KB;
+            int it = 0, s = 0;
+            uint32_t ph = 1;
+            unsigned long long w1 = 0;
+            for (; it < steps; ++it) {
+                if (!uniform_issue(mbar_wait<VOTE>(pk_empty(s), ph, abort_flag, 1, &w1))) break;
+                const uint32_t dst = base + Plan::kPkOff + s * Plan::kPkStage;
+                if (SOLO || elect_one()) {
+                    mbar_expect_tx(pk_full(s), Plan::kPkStage);
 #pragma unroll
-                for (int q = 0; q < KP; ++q) {
-                    tma_load_2d(dst + q * Plan::kPkBlock, &map_w, (kb + q) * (BK / 2), tile * BR, pk_full(s));
-                    tma_load_2d(dst + q * Plan::kPkBlock + BR * (BK / 2), &map_x, (kb + q) * (BK / 2), 0, pk_full(s));
+                    for (int q = 0; q < KP; ++q) {
+                        tma_load_2d(dst + q * Plan::kPkBlock, &map_w, (kb + q) * (BK / 2), tile * BR, pk_full(s));
+                        tma_load_2d(dst + q * Plan::kPkBlock + BR * (BK / 2), &map_x, (kb + q) * (BK / 2), 0, pk_full(s));
+                    }
                 }
+                if (!SOLO) __syncwarp();
+                if ((kb += KP) == KB) { kb = 0; ++tile; }
+                if (++s == SP) { s = 0; ph ^= 1; }
             }
-            __syncwarp();
-            if ((kb += KP) == KB) { kb = 0; ++tile; }
-            if (++s == SP) { s = 0; ph ^= 1; }
-        }
-        if (lane == 0) atomicAdd(&g_wait_ns[1], w1);
-        if (*abort_flag) {
-            // let the copies already issued land before the CTA leaves
-            for (int j = it > SP ? it - SP : 0; j < it; ++j) {
-                const uint64_t t0 = gtimer();
-                while (!mbar_try(pk_full(j % SP), (j / SP) & 1) && gtimer() - t0 < 100000000ull) {}
+            if (lane == 0) atomicAdd(&g_wait_ns[1], w1);
+            if (*abort_flag) {
+                // let the copies already issued land before the CTA leaves
+                for (int j = it > SP ? it - SP : 0; j < it; ++j) {
+                    const uint64_t t0 = gtimer();
+                    while (!mbar_try(pk_full(j % SP), (j / SP) & 1) && gtimer() - t0 < 100000000ull) {}
+                }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (the whole warp walks the loop, see elect_one)
-        // D s32; A = weights (signed), B = tokens (unsigned codes with zero-points, else signed); N = TOK, M = 128
-        const uint32_t idesc = (2u << 4) | (1u << 7) | ((A_UNSIGNED ? 0u : 1u) << 10) |
-                               ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(BR >> 4) << 24);
-        int kb = lin_begin % KB;
-        int u = 0, s = 0;
-        uint32_t ph = 0;
-        unsigned long long w2 = 0, w3 = 0;
-        for (int it = 0; it < steps; ++it) {
-            const int buf = u % NBUF;
-            const bool seg_first = it == 0 || kb == 0;
-            const bool seg_last = it == steps - 1 || kb == KB - KP;
-            bool ok = true;
-            if ((GROUPED || seg_first) && u >= NBUF) ok = mbar_wait(acc_empty(buf), ((u / NBUF) & 1) ^ 1, abort_flag, 2, &w2);
-            if (!ok || !mbar_wait(ex_full(s), ph, abort_flag, 3, &w3)) break;
-            tc_fence_after();
-            if (elect_one()) {
+        if (!SOLO || lane == 0) {
+            // ------------------------------------------------------------ MMA issuer
+            // D s32; A = weights (signed), B = tokens (unsigned codes with zero-points, else signed); N = TOK, M = 128
+            const uint32_t idesc = (2u << 4) | (1u << 7) | ((A_UNSIGNED ? 0u : 1u) << 10) |
+                                   ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(BR >> 4) << 24);
+            int kb = lin_begin % KB;
+            int u = 0, s = 0;
+            uint32_t ph = 0;
+            unsigned long long w2 = 0, w3 = 0;
+            for (int it = 0; it < steps; ++it) {
+                const int buf = u % NBUF;
+                const bool seg_first = it == 0 || kb == 0;
+                const bool seg_last = it == steps - 1 || kb == KB - KP;
+                bool ok = true;
+                if ((GROUPED || seg_first) && u >= NBUF) ok = mbar_wait<VOTE>(acc_empty(buf), ((u / NBUF) & 1) ^ 1, abort_flag, 2, &w2);
+                if (!uniform_issue(ok && mbar_wait<VOTE>(ex_full(s), ph, abort_flag, 3, &w3))) break;
+                tc_fence_after();
+                if (SOLO || elect_one()) {
 #pragma unroll
-                for (int q = 0; q < KP; ++q) {
-                    const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage + q * Plan::kExBlock;
-                    const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
+                    for (int q = 0; q < KP; ++q) {
+                        const uint32_t a_addr = base + Plan::kExOff + s * Plan::kExStage + q * Plan::kExBlock;
+                        const uint64_t adesc = make_smem_desc(a_addr), bdesc = make_smem_desc(a_addr + BR * BK);
 #pragma unroll
-                    for (int k4 = 0; k4 < BK / 32; ++k4) {
-                        const uint32_t accum = GROUPED ? (k4 > 0) : (!seg_first || k4 > 0);
-                        tc_mma_i8(tmem + (buf * KP + q) * TOK, adesc + 2 * k4, bdesc + 2 * k4, idesc, accum);
+                        for (int k4 = 0; k4 < BK / 32; ++k4) {
+                            const uint32_t accum = GROUPED ? (k4 > 0) : (!seg_first || k4 > 0);
+                            tc_mma_i8(tmem + (buf * KP + q) * TOK, adesc + 2 * k4, bdesc + 2 * k4, idesc, accum);
+                        }
                     }
+                    tc_commit(ex_empty(s));
+                    if (GROUPED || seg_last) tc_commit(acc_full(buf));
                 }
-                tc_commit(ex_empty(s));
-                if (GROUPED || seg_last) tc_commit(acc_full(buf));
+                if (!SOLO) __syncwarp();
+                if (GROUPED || seg_last) ++u;
+                if ((kb += KP) == KB) kb = 0;
+                if (++s == SE) { s = 0; ph ^= 1; }
             }
-            __syncwarp();
-            if (GROUPED || seg_last) ++u;
-            if ((kb += KP) == KB) kb = 0;
-            if (++s == SE) { s = 0; ph ^= 1; }
+            if (lane == 0) { atomicAdd(&g_wait_ns[2], w2); atomicAdd(&g_wait_ns[3], w3); }
         }
-        if (lane == 0) { atomicAdd(&g_wait_ns[2], w2); atomicAdd(&g_wait_ns[3], w3); }
     } else if (warp < 6) {
         // ------------------------------------------------------------ int4 -> int8 converters
         const int ct = tid - 64;                          // 0..127
@@ -234,8 +257,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         unsigned long long w4 = 0, w5 = 0;
         for (int it = 0; it < steps; ++it) {
             const int sp = it % SP, se = it % SE;
-            if (!mbar_wait(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4)) break;
-            if (!mbar_wait(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5)) break;
+            if (!uniform(mbar_wait<VOTE>(pk_full(sp), (it / SP) & 1, abort_flag, 4, &w4) &&
+                         mbar_wait<VOTE>(ex_empty(se), ((it / SE) & 1) ^ 1, abort_flag, 5, &w5))) break;
             const uint8_t *pk = sm + Plan::kPkOff + sp * Plan::kPkStage;
             uint8_t *ex = sm + Plan::kExOff + se * Plan::kExStage;
 #pragma unroll
@@ -258,8 +281,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
             fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) { mbar_arrive(ex_full(se)); mbar_arrive(pk_empty(sp)); }
+            meet();
+            if (arrives) { mbar_arrive(ex_full(se)); mbar_arrive(pk_empty(sp)); }
         }
         if (ct == 0) { atomicAdd(&g_wait_ns[4], w4); atomicAdd(&g_wait_ns[5], w5); }
     } else {
@@ -308,14 +331,13 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (GROUPED) {
                 // 256 * sum arrives from the tensor core; without zero-points the 1/256 rides in the weight scale
                 const float unit = A_UNSIGNED ? 1.0f : (1.0f / 256.0f);
-                const __half *bs = p.b_scale + (long)n * p.gb_cols;
-                const int32_t *br = A_UNSIGNED ? p.b_rowsum + (long)n * KB : nullptr;
+                // indexed from the parameters: two pointers kept for it cost 64 tokens with zero-points 1 - 2 %
                 float sbv[KP];
                 int rsv[KP];
 #pragma unroll
                 for (int q = 0; q < KP; ++q) {
-                    sbv[q] = __half2float(bs[gbs * (kb0 + q)]) * unit;
-                    rsv[q] = A_UNSIGNED ? br[kb0 + q] : 0;
+                    sbv[q] = __half2float((p.b_scale + (long)n * p.gb_cols)[gbs * (kb0 + q)]) * unit;
+                    rsv[q] = A_UNSIGNED ? (p.b_rowsum + (long)n * KB)[kb0 + q] : 0;
                 }
                 for (int kb = kb0; kb < kb1; kb += KP, ++u) {
                     float nsb[KP];
@@ -324,12 +346,12 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     for (int q = 0; q < KP; ++q) {       // the next step's channel data, fetched early
                         nsb[q] = sbv[q]; nrs[q] = rsv[q];
                         if (kb + KP < kb1) {
-                            if (gbs) nsb[q] = __half2float(bs[kb + KP + q]) * unit;
-                            if (A_UNSIGNED) nrs[q] = br[kb + KP + q];
+                            if (gbs) nsb[q] = __half2float((p.b_scale + (long)n * p.gb_cols)[kb + KP + q]) * unit;
+                            if (A_UNSIGNED) nrs[q] = (p.b_rowsum + (long)n * KB)[kb + KP + q];
                         }
                     }
                     const int buf = u % NBUF;
-                    ok = ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 6, &w6);
+                    ok = uniform(ok && mbar_wait<VOTE>(acc_full(buf), (u / NBUF) & 1, abort_flag, 6, &w6));
                     tc_fence_after();
 #pragma unroll
                     for (int q = 0; q < KP; ++q) {
@@ -337,8 +359,8 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                         if (ok) { tmem_ld_cols<TE>(tlane + (buf * KP + q) * TOK + j0, v); tc_wait_ld(); }
                         if (q == KP - 1) {
                             tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(acc_empty(buf));
+                            meet();
+                            if (arrives) mbar_arrive(acc_empty(buf));
                         }
                         if (ok) {
                             const float *sa = sa_s + gas * (kb + q) + j0;
@@ -359,13 +381,13 @@ gemm_decode_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             } else {
                 const int buf = u % NBUF;
-                ok = ok && mbar_wait(acc_full(buf), (u / NBUF) & 1, abort_flag, 7, &w6);
+                ok = uniform(ok && mbar_wait<VOTE>(acc_full(buf), (u / NBUF) & 1, abort_flag, 7, &w6));
                 tc_fence_after();
                 uint32_t v[TE];
                 if (ok) { tmem_ld_cols<TE>(tlane + buf * TOK + j0, v); tc_wait_ld(); }
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty(buf));
+                meet();
+                if (arrives) mbar_arrive(acc_empty(buf));
                 ++u;
 #pragma unroll
                 for (int j = 0; j < TE; ++j) acci[j] = ok ? (int)v[j] : 0;
