@@ -26,3 +26,24 @@ def test_decode_tc_steps_of_two_blocks(cuda, m, n, k, mode):
     assert ok, worst
     torch.cuda.synchronize()
     assert cuda.gemm_status()[0] == 0
+
+
+@pytest.mark.parametrize("m", [9, 16, 24, 32, 40, 64])
+@pytest.mark.parametrize("mode", [(128, 128, False), (128, 128, True), (0, 0, False), (0, 0, True)])
+def test_decode_tc_long_ranges(cuda, m, mode):
+    """28 K-blocks to a CTA (55 above 32 tokens): every ring of every form goes round several times.  The first and the last 384 channels (whole
+    tiles and shared ones) against the oracle."""
+    n, k = 16384, 8192
+    ap, bp, sa, sb, za, _ = make_case(m, m, n, k, *mode)
+    kw = dict(A_zero=None if za is None else _dev(za), B_rowsum=None if za is None else cuda.weight_rowsum(_dev(bp), mode[0] or k), algo=DECODE_TC)
+    d = cuda.gemm_i4_dequant(_dev(ap), _dev(bp), _dev(sa), _dev(sb), **kw)
+    for part in (slice(0, 384), slice(n - 384, n)):
+        want = O.gemm_i4_dequant(ap, bp[part], sa, sb[part], a_zero=za)
+        got = d[:, part].contiguous()
+        if mode[0] == 0:                                 # int32 sums: the split changes no bit
+            assert (got.cpu().numpy().view("u2") == want.view("u2")).all()
+        else:
+            ok, worst = _close(got, want)
+            assert ok, worst
+    torch.cuda.synchronize()
+    assert cuda.gemm_status()[0] == 0
