@@ -306,13 +306,15 @@ static int pick_stream(long M, long N, long K) {
 }
 
 // Batches with group-128 scales for which expanding both operands first pays for itself.  Both kernels walk whole waves of tiles
-// and both are bound by a time per 128-K block (measured on B200: 1.42 us for a wave of 148 tiles of 128 x 256 in the converting
-// kernel, 0.63 us for a wave of 74 pairs on 256 x 256 here); the expansion moves 1.5 bytes per code of either operand at 4.3 TB/s, and
-// the two launches cost 5 us more than one.  The estimate and the measurements agree on who wins, but for two shapes 2 % apart, in
-// the 102 of 65 to 8,192 rows, K = 1024 to 28672 and N = 256 to 57344 that were timed (us, converting / expanded): 256 rows 4096 -> 12288 46 / 37, 384
-// rows 47 / 58, 512 rows 90 / 58; 65 rows 11008 -> 4096 123 / 69; 65 rows 8192 -> 57344 182 / 279, 384 rows 483 / 399; 384 rows
-// 4096 -> 22016 90 / 88 (converting); 512 rows 1024 -> 8192 15 / 17; narrow outputs, where the rows are what is expanded: 8192 -> 256 with 8,192
-// rows 98 / 60, 4096 -> 512 46 / 33.
+// and both are bound by a time per 128-K block (B200: 1.42 us for a wave of 148 tiles of 128 x 256 in the converting kernel).  The
+// three terms of the expanded form are one fit to its two launches together (0.63 us for a wave of 74 pairs on 256 x 256, 0.35e-6 us per
+// code, 5 us).  Alone, from a cold cache, a wave of blocks takes 0.65 - 0.71 us, the expansion moves its 1.5 bytes per code at
+// 5.8 - 6.8 TB/s, and what is left beside them is 6 us; terms of those rates decide one of the timed shapes otherwise, by 4 %.
+// The estimate names the faster kernel for 107 of the 111 shapes that were timed (65 to 2,048 rows, 14 weights from 8192 -> 1280 to 8192 -> 57344,
+// operands from HBM, an idle GPU), and the other four are 1 - 5 % apart (us, converting / expanded): 256 rows 4096 -> 12288 50 / 39, 384 rows 51 / 60, 512 rows 95 / 61;
+// 65 rows 11008 -> 4096 121 / 67; 65 rows 8192 -> 57344 187 / 285, 384 rows 491 / 405; 384 rows 4096 -> 22016 96 / 92 and 128 to 384 rows
+// 1024 -> 8192 15.8 / 15.1 - 15.6 (both converting); narrow outputs, where the rows are what is expanded: 8192 -> 256 with 8,192 rows 98 / 60,
+// 4096 -> 512 46 / 33.
 static bool group_f8_pays(long M, long N, long K, long a_group, long b_group) {
     if ((a_group < b_group ? a_group : b_group) != 128 || K <= 128 || M <= 64 || !gemm_group_f8_supported(M, N, K)) return false;
     const long kb = K / 128, pairs = kNumSMs / 2;
@@ -324,7 +326,11 @@ int flh_b200_gemm_pick_algo(long M, long N, long K, long a_group, long b_group) 
     if ((a_group < b_group ? a_group : b_group) < 128) return FLH_B200_GEMM_MMA_SYNC;    // K-groups of 32 / 64
     if (M <= 64) return decode_tc_pays(M, N, K, a_group) ? FLH_B200_GEMM_DECODE_TC : pick_stream(M, N, K);
     // large batches without group scales: expanding both operands to int8 first pays for itself — from 1,536 rows, or from
-    // 1,024 when the output is wide enough to fill the GPU with 256 x 256 tiles (measured crossovers on B200)
+    // 1,024 when the output is wide enough to fill the GPU with 256 x 256 tiles.  The line is where an expansion at half of today's rate
+    // paid.  With today's (us, converting / expanded) it pays above the line almost everywhere (2,048 rows 4096 -> 12288 128 / 88, 1,024 rows
+    // 8192 -> 28672 262 / 211, but 1024 -> 8192 20 / 23), and below it already for 768 rows (4096 -> 22016 89 / 77, 8192 -> 8192 78 / 66) and for long
+    // rows on narrow outputs (65 to 1,024 rows 11008 -> 4096 51 / 46 to 54 / 52, 14336 -> 4096 65 / 56 to 67 / 62, 8192 -> 1280 37 / 34 to 38 / 35); not for
+    // 384 rows 4096 -> 12288 26 / 44, 8192 -> 28672 120 / 153, or 65 to 512 rows 8192 -> 8192 40 / 44 to 43 / 48.
     if (a_group == K && b_group == K && (M >= 1536 || (M >= 1024 && N >= 8192)))
         return N % 256 == 0 ? FLH_B200_GEMM_TCGEN05_I8_PAIR : FLH_B200_GEMM_TCGEN05_I8;
     return FLH_B200_GEMM_TCGEN05;

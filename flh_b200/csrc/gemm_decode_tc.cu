@@ -545,6 +545,8 @@ struct DecodeSplit { int tok, grid, per; };
 
 // Token columns, CTAs and K-blocks per CTA for a shape: as many CTAs as can be resident (two per SM up to 32
 // tokens, one above), never fewer than four K-blocks each unless the whole problem is smaller than that.
+// kp = 2: ranges of whole steps.  That can leave CTAs without work (64 tokens, 4096 -> 12288: 22 K-blocks on 140 CTAs in place of 21 on
+// 147, 23.6 us with single blocks, 22.1 so); of the shapes timed only 1024 -> 8192 lost by it (10.5, 10.7), where AUTO has another kernel.
 DecodeSplit decode_split(long M, long N, long K, int kp = 1) {
     DecodeSplit d;
     d.tok = M <= 16 ? 16 : (M <= 32 ? 32 : 64);

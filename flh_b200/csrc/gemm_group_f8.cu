@@ -12,9 +12,9 @@
 // A pair of CTAs (cta_group::2) shares one 256 x BN tile, as in gemm_i8.cu: 64 KB of shared-memory traffic per CTA and
 // block instead of 96.  Per block the MMA thread fills one of two TMEM buffers while the epilogue warps fold the other.
 //
-// Measured (B200, expansion included): 2048 x 4096 -> 12288 146 us, 4096 -> 22016 235 us, 11008 -> 4096 130 us; the converting kernel
-// of gemm_tcgen05.cu, which has the same results, 266, 439 and 247 us.  The epilogue is the limit, and of its time what it spends on
-// barriers counts most.  For the first shape: eight epilogue warps and issue loops walked by one lane 183; sixteen warps 179; their
+// Measured (B200, expansion included, operands from HBM): 2048 x 4096 -> 12288 149 us, 4096 -> 22016 243 us, 11008 -> 4096 132 us; the
+// converting kernel of gemm_tcgen05.cu, which has the same results, 272, 445 and 256 us.  The epilogue is the limit, and of its time what
+// it spends on barriers counts most.  For the first shape, the same operands call after call: eight epilogue warps and issue loops walked by one lane 183; sixteen warps 179; their
 // wait and arrival for the scales of every fourth K-block in place of each 157; waits with one outcome for the warp (mbar_wait_warp)
 // and the leader's barrier mapped once 146.
 //

@@ -245,7 +245,10 @@ class LinearFLH(torch.nn.Module):
             self._rowsum = _CUDA.weight_rowsum(self.w_packed.view(self.out_features, self.in_features // 2), group)
         return self._rowsum
 
-    PREPACK_MIN_ROWS = 256      # batches from which the int8 copy is used
+    # Batches from which the int8 copy is used.  B200, us, converting / with the copy: 256 rows 4096 -> 12288 26 / 23, 4096 -> 22016 47 / 34,
+    # 8192 -> 28672 84 / 60, but a few shapes above it lose (384 rows 4096 -> 12288 26 / 31, 8192 -> 10240 43 / 50); 128 rows win on the
+    # narrower outputs (8192 -> 8192 41 / 30) and lose on the wide ones (4096 -> 22016 27 / 33, 8192 -> 28672 46 / 58).
+    PREPACK_MIN_ROWS = 256
 
     def prepack_int8(self):
         """Keep an int8 copy of the weights (1 byte per weight on top of the packed half byte) for large-batch
